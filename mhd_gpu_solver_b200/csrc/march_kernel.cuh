@@ -105,11 +105,15 @@ __device__ __forceinline__ double march_strip(const typename Policy::Args& a, in
         prim(y0 - 1, r1, wb);
         prim(y0, r2, Wm);
         prim(y0 + 1, r3, Wp);
+        T d0[9], d1[9], d2[9];
 #pragma unroll
         for (int c = 0; c < 9; ++c) {
-            sYm[c] = limit_slope<L>(wb[c] - wa[c], Wm[c] - wb[c]);
-            sYc[c] = limit_slope<L>(Wm[c] - wb[c], Wp[c] - Wm[c]);
+            d0[c] = wb[c] - wa[c];
+            d1[c] = Wm[c] - wb[c];
+            d2[c] = Wp[c] - Wm[c];
         }
+        limit_half_slopes<L>(d0, d1, sYm);
+        limit_half_slopes<L>(d1, d2, sYc);
         face_flux_regs<T, true>(wb, sYm, Wm, sYc, gamma, inv_gm1, c_h, Gm);
         if constexpr (NI) {
             T Jb[3];
@@ -125,14 +129,14 @@ __device__ __forceinline__ double march_strip(const typename Policy::Args& a, in
         // x sweep of row y: dF = F(x + 1/2) - F(x - 1/2) on the owned lanes
         T dF[9];
         {
-            T Wn[9], sX[9], sXn[9], F[9];
+            T Wn[9], sX[9], sXn[9], F[9], dL[9], dR[9];
 #pragma unroll
             for (int c = 0; c < 9; ++c) {
                 Wn[c] = __shfl_down_sync(kFull, Wm[c], 1);
-                const T dR = Wn[c] - Wm[c];
-                const T dL = __shfl_up_sync(kFull, dR, 1);
-                sX[c] = limit_slope<L>(dL, dR);
+                dR[c] = Wn[c] - Wm[c];
+                dL[c] = __shfl_up_sync(kFull, dR[c], 1);
             }
+            limit_half_slopes<L>(dL, dR, sX);
 #pragma unroll
             for (int c = 0; c < 9; ++c) {
                 sXn[c] = __shfl_down_sync(kFull, sX[c], 1);
@@ -149,12 +153,14 @@ __device__ __forceinline__ double march_strip(const typename Policy::Args& a, in
         // row y+3 in flight while row y+2 is converted and the y face y+1/2 is evaluated
         Raw rq;
         load(y + 3, rq);
-        T W2[9], sYn[9], Gp[9];
+        T W2[9], sYn[9], Gp[9], dm[9], dp[9];
         prim(y + 2, rn, W2);
 #pragma unroll
         for (int c = 0; c < 9; ++c) {
-            sYn[c] = limit_slope<L>(Wp[c] - Wm[c], W2[c] - Wp[c]);
+            dm[c] = Wp[c] - Wm[c];
+            dp[c] = W2[c] - Wp[c];
         }
+        limit_half_slopes<L>(dm, dp, sYn);
         face_flux_regs<T, true>(Wm, sYc, Wp, sYn, gamma, inv_gm1, c_h, Gp);
         T Jn[NI ? 3 : 1];
         if constexpr (NI) {

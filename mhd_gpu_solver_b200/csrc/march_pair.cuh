@@ -183,7 +183,7 @@ __device__ __forceinline__ double march_pair_strip(const StageArgsDelta& a, cons
                 sYm[j][c] = limit_half_slope<L>(wb[j][c] - wa[j][c], Wm[j][c] - wb[j][c]);
                 sYc[j][c] = limit_half_slope<L>(Wm[j][c] - wb[j][c], Wp[j][c] - Wm[j][c]);
             }
-            face_flux_regs<T, true, true>(wb[j], sYm[j], Wm[j], sYc[j], gamma, inv_gm1, c_h,
+            face_flux_regs<T, true>(wb[j], sYm[j], Wm[j], sYc[j], gamma, inv_gm1, c_h,
                                           Gm[j]);
         }
         if constexpr (NI) {
@@ -262,8 +262,8 @@ __device__ __forceinline__ double march_pair_strip(const StageArgsDelta& a, cons
             for (int c = 0; c < 9; ++c) {
                 sAn[c] = __shfl_down_sync(kFull, sA[c], 1);
             }
-            face_flux_regs<T, false, true>(Wm[0], sA, Wm[1], sB, gamma, inv_gm1, c_h, FA);
-            face_flux_regs<T, false, true>(Wm[1], sB, An, sAn, gamma, inv_gm1, c_h, FB);
+            face_flux_regs<T, false>(Wm[0], sA, Wm[1], sB, gamma, inv_gm1, c_h, FA);
+            face_flux_regs<T, false>(Wm[1], sB, An, sAn, gamma, inv_gm1, c_h, FB);
             if constexpr (NI) {
                 const T jx = __shfl_down_sync(kFull, Jc[0][0], 1);
                 const T jy = __shfl_down_sync(kFull, Jc[0][1], 1);
@@ -289,7 +289,7 @@ __device__ __forceinline__ double march_pair_strip(const StageArgsDelta& a, cons
             for (int c = 0; c < 9; ++c) {
                 sYn[j][c] = limit_half_slope<L>(Wp[j][c] - Wm[j][c], W2[j][c] - Wp[j][c]);
             }
-            face_flux_regs<T, true, true>(Wm[j], sYc[j], Wp[j], sYn[j], gamma, inv_gm1, c_h,
+            face_flux_regs<T, true>(Wm[j], sYc[j], Wp[j], sYn[j], gamma, inv_gm1, c_h,
                                           Gp[j]);
         }
         if constexpr (NI) {

@@ -278,7 +278,7 @@ __device__ __forceinline__ double march_tma_strip(const typename Policy::Args& a
             limit_half_slopes<L>(d0, d1, sYm);
             limit_half_slopes<L>(d1, d2, sYc);
         }
-        face_flux_regs<T, true, true>(wb, sYm, Wm, sYc, gamma, inv_gm1, c_h, Gm);
+        face_flux_regs<T, true>(wb, sYm, Wm, sYc, gamma, inv_gm1, c_h, Gm);
         if constexpr (Lay::kStash) {
             // the own cells' delta of rows y0 and y0 + 1 (the ring's first two items)
             if (own) {
@@ -327,7 +327,7 @@ __device__ __forceinline__ double march_tma_strip(const typename Policy::Args& a
             for (int c = 0; c < 9; ++c) {
                 sXn[c] = __shfl_down_sync(kFull, sX[c], 1);
             }
-            face_flux_regs<T, false, true>(Wm, sX, Wn, sXn, gamma, inv_gm1, c_h, F);
+            face_flux_regs<T, false>(Wm, sX, Wn, sXn, gamma, inv_gm1, c_h, F);
             if constexpr (NI) {
                 march_nonideal_x(Jc, Wm, Wn, k.ni, F);
             }
@@ -389,7 +389,7 @@ __device__ __forceinline__ double march_tma_strip(const typename Policy::Args& a
             }
             limit_half_slopes<L>(dm, dp, sYn);
         }
-        face_flux_regs<T, true, true>(Wm, sYc, Wp, sYn, gamma, inv_gm1, c_h, Gp);
+        face_flux_regs<T, true>(Wm, sYc, Wp, sYn, gamma, inv_gm1, c_h, Gp);
         T Jn[NI ? 3 : 1];
         if constexpr (NI) {
             march_current(Wm, Wp, W2, inv_2dx, inv_2dy, Jn);

@@ -58,9 +58,10 @@ constexpr size_t stage_smem_bytes()
     return sizeof(T) * (9 * S::NH + 9 * slopes + 9 * fluxes + (NI ? 3 * S::NJ : 0));
 }
 
-// One cell of a slope sweep: per component the limited slope s = lim(W - W_prev, W_next - W)
-// (include/mhd/kernels/muscl_hll.hpp:64-65), stored at sS[c * sn + t]. Sweep regions: x: columns
-// 1..TX+2 and rows 2..TY+1 of the halo tile; y: columns 2..TX+1 and rows 1..TY+2.
+// One cell of a slope sweep: per component half the limited slope, s = lim(W - W_prev,
+// W_next - W) / 2 (include/mhd/kernels/muscl_hll.hpp:64-67), stored at sS[c * sn + t]. Sweep
+// regions: x: columns 1..TX+2 and rows 2..TY+1 of the halo tile; y: columns 2..TX+1 and rows
+// 1..TY+2.
 template <int L, class T, int TX, int TY, bool YDIR>
 __device__ __forceinline__ void slope_item(const T* __restrict__ sW, T* __restrict__ sS, int sn,
                                            int t)
@@ -71,29 +72,18 @@ __device__ __forceinline__ void slope_item(const T* __restrict__ sW, T* __restri
     constexpr int step = YDIR ? HX : 1;
     const int sx = t % W, sy = t / W;
     const int i = YDIR ? (sy + 1) * HX + (sx + 2) : (sy + 2) * HX + (sx + 1);
-    if constexpr (L == kVanLeer && sizeof(T) == 8) {
-        // the nine components at once: one division (limit_half_slopes), slope = 2 x half
-        // slope (exact)
-        T dm[9], dp[9], h[9];
+    T dm[9], dp[9], h[9];
 #pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            const T* w = sW + c * S::NH + i;
-            const T wm = w[-step], w0 = w[0], wp = w[step];
-            dm[c] = w0 - wm;
-            dp[c] = wp - w0;
-        }
-        limit_half_slopes<L>(dm, dp, h);
+    for (int c = 0; c < 9; ++c) {
+        const T* w = sW + c * S::NH + i;
+        const T wm = w[-step], w0 = w[0], wp = w[step];
+        dm[c] = w0 - wm;
+        dp[c] = wp - w0;
+    }
+    limit_half_slopes<L>(dm, dp, h);
 #pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            sS[c * sn + t] = T(2) * h[c];
-        }
-    } else {
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            const T* w = sW + c * S::NH + i;
-            const T wm = w[-step], w0 = w[0], wp = w[step];
-            sS[c * sn + t] = limit_slope<L>(w0 - wm, wp - w0);
-        }
+    for (int c = 0; c < 9; ++c) {
+        sS[c * sn + t] = h[c];
     }
 }
 
@@ -107,33 +97,49 @@ __device__ __forceinline__ void face_states(const T* __restrict__ sW, T* __restr
     }
 }
 
-// One face flux from the centre values lc, rc and limited slopes sl, sr (physical component
-// order) of its two cells: left state W(l) + s(l)/2, right state W(r) - s(r)/2
+// One face flux from the centre values lc, rc and half limited slopes sl, sr (physical component
+// order) of its two cells: left state W(l) + s(l), right state W(r) - s(r)
 // (include/mhd/kernels/muscl_hll.hpp:66-67), with the both-sides first-order fallback of
-// muscl_hll.hpp:145-168. Output in physical component order. HALF: sl and sr hold half slopes
-// s/2 (exact halves), so the face states are W(l) + s'(l) and W(r) - s'(r), the same values.
-template <class T, bool YDIR, bool HALF = false>
+// muscl_hll.hpp:145-168. Output in physical component order.
+template <class T, bool YDIR>
 __device__ __forceinline__ void face_flux_regs(const T (&lc)[9], const T (&sl)[9],
                                                const T (&rc)[9], const T (&sr)[9], T gamma,
                                                T inv_gm1, T c_h, T (&out)[9])
 {
     // physical component feeding each rotated-frame slot (rho, vn, vt, vz, p, bn, bt, bz, psi)
     constexpr int comp[9] = {0, YDIR ? 2 : 1, YDIR ? 1 : 2, 3, 4, YDIR ? 6 : 5, YDIR ? 5 : 6, 7, 8};
-    // Density and pressure of both states decide the fallback; then every component is
-    // W + h s with h = 1/2 (second order) or h = 0 (first order: W + 0 s = W exactly for finite
-    // slopes, and 0.5 s is exact, so both cases give the reference's values).
-    const T inf = T(INFINITY);
-    const T hs = HALF ? T(1) : T(0.5);
-    const T l0 = lc[0] + hs * sl[0], l4 = lc[4] + hs * sl[4];
-    const T r0 = rc[0] - hs * sr[0], r4 = rc[4] - hs * sr[4];
-    const bool ok = (l0 > T(0)) && (l4 > T(0)) && (l0 < inf) && (l4 < inf) && (r0 > T(0)) &&
-                    (r4 > T(0)) && (r0 < inf) && (r4 < inf);
-    const T h = ok ? hs : T(0);
     T l[9], r[9];
+    if constexpr (sizeof(T) == 8) {
+        // The second-order states, and the first-order ones only where a density or pressure
+        // fails the test.
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        l[q] = lc[comp[q]] + h * sl[comp[q]];
-        r[q] = rc[comp[q]] - h * sr[comp[q]];
+        for (int q = 0; q < 9; ++q) {
+            l[q] = lc[comp[q]] + sl[comp[q]];
+            r[q] = rc[comp[q]] - sr[comp[q]];
+        }
+        if (!(positive_finite(l[0]) && positive_finite(l[4]) && positive_finite(r[0]) &&
+              positive_finite(r[4]))) {
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                l[q] = lc[comp[q]];
+                r[q] = rc[comp[q]];
+            }
+        }
+    } else {
+        // Density and pressure of both states decide the fallback; then every component is
+        // W + h s with h = 1 (second order) or h = 0 (first order: W + 0 s = W exactly for finite
+        // slopes).
+        const T l0 = lc[0] + sl[0], l4 = lc[4] + sl[4];
+        const T r0 = rc[0] - sr[0], r4 = rc[4] - sr[4];
+        const T inf = T(INFINITY);
+        const bool ok = (l0 > T(0)) && (l4 > T(0)) && (l0 < inf) && (l4 < inf) && (r0 > T(0)) &&
+                        (r4 > T(0)) && (r0 < inf) && (r4 < inf);
+        const T h = ok ? T(1) : T(0);
+#pragma unroll
+        for (int q = 0; q < 9; ++q) {
+            l[q] = lc[comp[q]] + h * sl[comp[q]];
+            r[q] = rc[comp[q]] - h * sr[comp[q]];
+        }
     }
     const PrimN<T> WL{l[0], l[1], l[2], l[3], l[4], l[5], l[6], l[7], l[8]};
     const PrimN<T> WR{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8]};
@@ -286,7 +292,7 @@ __device__ __forceinline__ double stage_tile(const typename Policy::Args& a, int
     constexpr int R = (TX * TY + NT - 1) / NT; // owned cells per thread
     const Ctrl* __restrict__ ctrl = a.ctrl;
     T* sW = reinterpret_cast<T*>(smem_raw); // [9][HY][HX] primitives
-    T* sS = sW + 9 * S::NH;                 // [9][SN] limited slopes of the current sweep
+    T* sS = sW + 9 * S::NH;                 // [9][SN] half limited slopes of the current sweep
     T* sF = sS + 9 * S::SN;                 // [9][NF] face fluxes
     T* sJ = sF + 9 * S::NF;                 // [3][JY][JX] current
 
