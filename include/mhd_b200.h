@@ -197,13 +197,14 @@ int mhdb_tile_config_count(int precision);
 int mhdb_tile_config_info(int precision, int config, int* tile_x, int* tile_y, int* threads,
                           int* min_blocks);
 int mhdb_tile_config_kind(int precision, int config);
-/* mhdb_set_tile_config(h, -1) restores the default: FP32-mixed solves of at least 1024 x 1024
-   cells run the TMA strip march (one warp per block; unmasked solves in the increment form,
-   configuration 13; masked ones configuration 11, the TMA strip march that also serves masks),
-   smaller FP32-mixed ones configuration 0; FP64 solves of
-   at least 2048 x 2048 cells run the FP64 TMA strip march (configuration 7, which also serves
-   masks), smaller ones the 320-thread tile kernel (configuration 2, non-ideal ones configuration
-   0), smaller masked FP64 solves configuration 0. */
+/* mhdb_set_tile_config(h, -1) restores the default, by the grid's cells: unmasked FP32-mixed solves
+   run the TMA strip march of the increment form (configuration 17) from 768 x 768 cells up and the
+   one-warp register march (configuration 18) below; masked ones the TMA strip march that also
+   serves masks (configuration 11) from 1024 x 1024 up and configuration 0 below. Unmasked FP64
+   solves run the FP64 TMA strip march (configuration 7), between about 190 x 190 and 264 x 264
+   cells the 320-thread tile kernel (configuration 2; non-ideal ones configuration 0); masked ones
+   configuration 7 from 2048 x 2048 up and configuration 0 below. The strip marches cut a grid into
+   segments of at most their tile height, by the size of the grid. */
 int mhdb_set_tile_config(mhdb_solver* h, int config);
 
 /* Additive, for tests of the error path: every bulk-copy wait of the TMA strip marches is bounded
@@ -298,7 +299,7 @@ int mhdb_batch_poll(mhdb_batch* b, int* active);
    (tile width and height), its threads and its kernel kind (MHDB_KERNEL_*). FP32-mixed: 0 = TMA
    strip march, one warp by 32 rows; 1 = register strip march, 4 warps by 32 rows; 2 = TMA strip
    march, one warp by 64 rows; 3 = TMA strip march of the increment form, one warp by 32 rows
-   (the default for solves of at least 128 x 128 cells; smaller ones take 1).
+   (the default). Solves of fewer than 128 x 128 cells take 16 rows in place of 32.
    mhdb_batch_set_config picks one for a solve (-1: by the solve's size, the default); once a
    solve has been stepped it cannot change between configuration 3 and the others
    (MHDB_INVALID_ARGUMENT). The batch autotuner (mhd_gpu_solver_b200.autotune.tune_batch) chooses

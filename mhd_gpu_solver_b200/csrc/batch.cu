@@ -194,6 +194,17 @@ struct BatchVariant {
     int tile_x, tile_y, threads, kind; // kind: MHDB_KERNEL_*
 };
 
+// Rows of a solve's work items. A march item is a serial chain of its rows: a batch of a few small
+// solves ends with its longest chain (64 solves of 64^2, per step: 32-row items 128 us, 16-row ones
+// 83), a full one pays for finer items' prologues (64 solves of sides 64-1024: 916 us with 32 rows,
+// 1056 with 16 below 1024^2). The rule sees the solve alone, never the mix: a solve's values do not
+// depend on the other solves.
+int item_rows(const BatchVariant& v, const mhdb_grid& g)
+{
+    const long long cells = static_cast<long long>(g.nx) * g.ny;
+    return v.tile_y == 32 && cells < 128LL * 128 ? 16 : v.tile_y;
+}
+
 template <class Policy>
 struct BatchKernels;
 
@@ -238,16 +249,17 @@ struct BatchKernels<PolicyMixed> {
         if (v == 3) return {kMarchOwned, 32, 32, MHDB_KERNEL_MARCH_TMA_DELTA};
         return {kMarchOwned, 32, 32, MHDB_KERNEL_MARCH_TMA};
     }
-    // Small solves have too few strips to fill the GPU on their own; their per-item set-up is
-    // cheaper in the register march. Larger ones run the increment form.
-    static int default_variant(long long cells) { return cells >= 128LL * 128 ? 3 : 1; }
+    // The increment form for every size: lists of one configuration share a launch per stage, so a
+    // small solve's items run beside the others' (in the register march of configuration 1, and a
+    // launch of its own, one solve under 128^2 cells cost 180 us per step).
+    static int default_variant(long long) { return kDeltaVariant; }
     template <int L, bool NI, int STAGE>
     static Fn fn(int v)
     {
-        if (v == 1) return batch_march_kernel<PolicyMixed, L, NI, STAGE, 32, 4, 4, BatchSolveTma>;
-        if (v == 2) return batch_march_tma_kernel<L, NI, STAGE, 64, 1, 16, true, (STAGE == 1 ? 1 : 0)>;
-        if (v == 3) return batch_march_delta_kernel<L, NI, STAGE, 32, 1, 16, true>;
-        return batch_march_tma_kernel<L, NI, STAGE, 32, 1, 16, true, (STAGE == 1 ? 1 : 0)>;
+        if (v == 1) return batch_march_kernel<PolicyMixed, L, NI, STAGE, 4, 4, BatchSolveTma>;
+        if (v == 2) return batch_march_tma_kernel<L, NI, STAGE, 1, 16, true, (STAGE == 1 ? 1 : 0)>;
+        if (v == 3) return batch_march_delta_kernel<L, NI, STAGE, 1, 16, true>;
+        return batch_march_tma_kernel<L, NI, STAGE, 1, 16, true, (STAGE == 1 ? 1 : 0)>;
     }
     static size_t smem(int v, bool, int stage)
     {
@@ -291,7 +303,7 @@ struct SolveRec {
     int slot = -1;
     int config = -1;  // batch configuration chosen for this solve (-1: from its size)
     int variant = 0;  // configuration in use (set when the work lists are built)
-    int tiles_x = 0, tiles_y = 0;
+    int tiles_x = 0, tiles_y = 0, rows = 0; // rows: of a work item
     bool fixed = false;
     Ctrl last{}; // host copy after the last poll
     MarchTmaMaps maps[2]{}; // FP32-mixed: tensor maps of stage 1 and stage 2
@@ -405,6 +417,7 @@ void rebuild(mhdb_batch* b)
     using K = BatchKernels<Policy>;
     using Desc = typename K::Desc;
     std::vector<Desc> descs;
+    std::vector<int> rows; // of a work item, by descriptor
     std::map<std::tuple<int, int, int>, std::vector<int2>> items; // (variant, limiter, ni)
     for (size_t id = 0; id < b->solves.size(); ++id) {
         SolveRec& s = b->solves[id];
@@ -416,18 +429,19 @@ void rebuild(mhdb_batch* b)
                         : K::default_variant(static_cast<long long>(s.grid.nx) * s.grid.ny);
         const BatchVariant bv = K::variant(s.variant);
         s.tiles_x = (s.grid.nx + bv.tile_x - 1) / bv.tile_x;
-        s.tiles_y = (s.grid.ny + bv.tile_y - 1) / bv.tile_y;
+        s.rows = item_rows(bv, s.grid);
+        s.tiles_y = (s.grid.ny + s.rows - 1) / s.rows;
         Desc d{};
         Ctrl* ctrl = b->ctrl + s.slot;
         if constexpr (sizeof(typename Policy::T) == 8) {
             d.stage[0] = StageArgsF64{static_cast<const double*>(s.U), static_cast<double*>(s.Us),
-                                      nullptr, ctrl, s.geom, s.k, 1};
+                                      nullptr, ctrl, s.geom, s.k, 1, s.rows};
             d.stage[1] = StageArgsF64{static_cast<const double*>(s.Us), static_cast<double*>(s.U),
-                                      nullptr, ctrl, s.geom, s.k, 1};
+                                      nullptr, ctrl, s.geom, s.k, 1, s.rows};
         } else {
             const MixedState u = mixed_view(s.U, s.geom), us = mixed_view(s.Us, s.geom);
-            d.stage[0] = StageArgsMx{u, us, nullptr, ctrl, s.geom, s.k, 1};
-            d.stage[1] = StageArgsMx{us, u, nullptr, ctrl, s.geom, s.k, 1};
+            d.stage[0] = StageArgsMx{u, us, nullptr, ctrl, s.geom, s.k, 1, s.rows};
+            d.stage[1] = StageArgsMx{us, u, nullptr, ctrl, s.geom, s.k, 1, s.rows};
             d.maps[0] = s.maps[0];
             d.maps[1] = s.maps[1];
             const bool alt = s.variant == BatchKernels<PolicyMixed>::kDeltaVariant;
@@ -453,7 +467,7 @@ void rebuild(mhdb_batch* b)
                 const MixedState bufs[2] = {u, us};
                 for (int q = 0; q < 2; ++q) {
                     d.dstage[q] = StageArgsDelta{bufs[q], bufs[1 - q], s.delta, nullptr, ctrl,
-                                                 s.geom, s.k, 1};
+                                                 s.geom, s.k, 1, s.rows};
                     d.dmaps[q][0] = s.dmaps[q][0];
                     d.dmaps[q][1] = s.dmaps[q][1];
                 }
@@ -463,10 +477,17 @@ void rebuild(mhdb_batch* b)
         d.ntiles = s.tiles_x * s.tiles_y;
         const int di = static_cast<int>(descs.size());
         descs.push_back(d);
+        rows.push_back(s.rows);
         auto& v = items[{s.variant, s.limiter, s.ni ? 1 : 0}];
         for (int t = 0; t < d.ntiles; ++t) {
             v.push_back(make_int2(di, t));
         }
+    }
+    // Long items first: the CTAs walk a list with a grid stride, so the short ones even out the end.
+    for (auto& kv : items) {
+        std::stable_sort(kv.second.begin(), kv.second.end(), [&](const int2& a, const int2& b) {
+            return rows[a.x] > rows[b.x];
+        });
     }
     std::vector<int2> work;
     b->lists.clear();

@@ -37,14 +37,15 @@ void fill_pair_tile(StageKernels& k)
     k.smem2 = k.smem;
 }
 
-// Strip-march configuration: NW warps per block, LY rows per warp, MINB blocks per SM.
+// Strip-march configuration: NW warps per block, at most LY rows per warp, MINB blocks per SM.
 template <int NW_, int LY_, int MINB_>
 struct MarchCfg {
     static constexpr int NW = NW_, LY = LY_, MINB = MINB_;
     static constexpr bool MARCH = true;
 };
 
-// TMA-fed strip-march configuration: NW warps per block, LY rows per warp, MINB blocks per SM.
+// TMA-fed strip-march configuration: NW warps per block, at most LY rows per warp, MINB blocks
+// per SM.
 template <int NW_, int LY_, int MINB_, bool HF_ = true, int ST1_ = 1, int ST2_ = 0,
           int DELTA_ = 0>
 struct MarchTmaCfg {
@@ -104,23 +105,25 @@ void fill_pair(StageKernels& k)
         if constexpr (E == 8) {
             static_assert(Cfg::ST1 == 0 && Cfg::ST2 == 0,
                           "the FP64 TMA strip march stores through the lanes");
-            k.f64_tma1 = march_tma_kernel<L, 1, Cfg::LY, Cfg::NW, Cfg::MINB, Cfg::HF, 0, NI, MASK,
+            k.f64_tma1 = march_tma_kernel<L, 1, Cfg::NW, Cfg::MINB, Cfg::HF, 0, NI, MASK,
                                           Policy>;
-            k.f64_tma2 = march_tma_kernel<L, 2, Cfg::LY, Cfg::NW, Cfg::MINB, Cfg::HF, 0, NI, MASK,
+            k.f64_tma2 = march_tma_kernel<L, 2, Cfg::NW, Cfg::MINB, Cfg::HF, 0, NI, MASK,
                                           Policy>;
         } else if constexpr (Cfg::DELTA) {
             static_assert(Cfg::ST1 == 0 && Cfg::ST2 == 0, "the increment form stores through the lanes");
-            k.dx_tma1 = march_tma_kernel<L, 1, Cfg::LY, Cfg::NW, Cfg::MINB, Cfg::HF, 0, NI, MASK,
+            k.dx_tma1 = march_tma_kernel<L, 1, Cfg::NW, Cfg::MINB, Cfg::HF, 0, NI, MASK,
                                          PolicyDelta<1>>;
-            k.dx_tma2 = march_tma_kernel<L, 2, Cfg::LY, Cfg::NW, Cfg::MINB, Cfg::HF, 0, NI, MASK,
+            k.dx_tma2 = march_tma_kernel<L, 2, Cfg::NW, Cfg::MINB, Cfg::HF, 0, NI, MASK,
                                          PolicyDelta<2, Cfg::DELTA>>;
         } else {
-            k.mx_tma1 = march_tma_kernel<L, 1, Cfg::LY, Cfg::NW, Cfg::MINB, Cfg::HF, Cfg::ST1, NI, MASK>;
-            k.mx_tma2 = march_tma_kernel<L, 2, Cfg::LY, Cfg::NW, Cfg::MINB, Cfg::HF, Cfg::ST2, NI, MASK>;
+            k.mx_tma1 = march_tma_kernel<L, 1, Cfg::NW, Cfg::MINB, Cfg::HF, Cfg::ST1, NI, MASK>;
+            k.mx_tma2 = march_tma_kernel<L, 2, Cfg::NW, Cfg::MINB, Cfg::HF, Cfg::ST2, NI, MASK>;
         }
         constexpr int K = Cfg::DELTA;
         k.tile_x = Cfg::NW * kMarchOwned;
         k.tile_y = Cfg::LY;
+        k.segments = true;
+        k.min_blocks = E == 8 && Cfg::NW == 1 && Cfg::MINB == 10 ? 12 : Cfg::MINB; // 168 registers fit 12
         k.threads = Cfg::NW * 32;
         k.smem = march_tma_smem_bytes<1, Cfg::ST1, E, (K > 0 ? 1 : 0)>(Cfg::NW);
         k.smem2 = march_tma_smem_bytes<2, Cfg::ST2, E, K>(Cfg::NW);
@@ -128,8 +131,8 @@ void fill_pair(StageKernels& k)
     } else if constexpr (is_march<Cfg>::value) {
         static_assert(!MASK, "the strip-march kernel serves unmasked solves");
         using T = typename Policy::T;
-        auto s1 = march_kernel<Policy, L, 1, Cfg::LY, Cfg::NW, Cfg::MINB, NI>;
-        auto s2 = march_kernel<Policy, L, 2, Cfg::LY, Cfg::NW, Cfg::MINB, NI>;
+        auto s1 = march_kernel<Policy, L, 1, Cfg::NW, Cfg::MINB, NI>;
+        auto s2 = march_kernel<Policy, L, 2, Cfg::NW, Cfg::MINB, NI>;
         if constexpr (sizeof(T) == 8) {
             k.f64_stage1 = s1;
             k.f64_stage2 = s2;
@@ -139,6 +142,8 @@ void fill_pair(StageKernels& k)
         }
         k.tile_x = Cfg::NW * kMarchOwned;
         k.tile_y = Cfg::LY;
+        k.segments = true;
+        k.min_blocks = Cfg::MINB;
         k.threads = Cfg::NW * 32;
         k.smem = 0;
         k.smem2 = 0;

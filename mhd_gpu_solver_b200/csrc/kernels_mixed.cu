@@ -23,6 +23,7 @@ using Cfg15 = MarchPairCfg<32, 8>;  // increment form, two columns per lane
 using Cfg16 = MarchPairCfg<32, 10>; // the same, 10 blocks per SM requested (168 registers)
 // increment form, stage 2's own-cell delta from the halo stream (also masked)
 using Cfg17 = MarchTmaCfg<1, 32, 16, true, 0, 0, 2>;
+using Cfg18 = MarchCfg<1, 32, 16>; // one-warp register march (stored form)
 constexpr TileConfigInfo kInfo[] = {
     {32, 16, 256, 2, kKindTile},       {32, 16, 256, 3, kKindTile},
     {32, 8, 256, 3, kKindTile},        {32, 16, 384, 2, kKindTileMerged},
@@ -32,20 +33,27 @@ constexpr TileConfigInfo kInfo[] = {
     {112, 32, 128, 4, kKindMarchTma},  {28, 32, 32, 16, kKindMarchTma},
     {28, 64, 32, 16, kKindMarchTma},   {28, 32, 32, 16, kKindMarchTmaDelta},
     {28, 64, 32, 16, kKindMarchTmaDelta}, {60, 32, 32, 8, kKindMarchTmaPair},
-    {60, 32, 32, 10, kKindMarchTmaPair}, {28, 32, 32, 16, kKindMarchTmaDelta}};
+    {60, 32, 32, 10, kKindMarchTmaPair}, {28, 32, 32, 16, kKindMarchTmaDelta},
+    {28, 32, 32, 16, kKindMarch}};
 constexpr int kCount = sizeof(kInfo) / sizeof(kInfo[0]);
 } // namespace
 
 int stage_config_count_mixed() { return kCount; }
 
-// Without a chosen configuration: grids of at least 1024^2 cells run the TMA strip march with one
-// warp per block, unmasked ones in the increment form with stage 2's own-cell increment taken
-// from the halo stream (configuration 17), masked ones in the stored form that also serves masks
-// (configuration 11); smaller grids have too few 28-column strips to fill the GPU with it and run
-// the shared-memory tile kernel.
+// Without a chosen configuration: unmasked grids of at least 768^2 cells run the TMA strip march of
+// the increment form with stage 2's own-cell increment taken from the halo stream (configuration
+// 17); smaller ones, whose state stays in L2, the one-warp register march of the stored form
+// (configuration 18), which has no copies to set up (per step, register against TMA march: 128^2
+// 13.4 and 14.3, 360^2 22.2 and 25.2, 512^2 38 and 39, 640^2 49 and 50, 724^2 56 and 56, 900^2 90
+// and 84, 1024^2 110 and 99 us; the tile kernel took 18.5, 24.9, 46 and 168 us at 128^2, 360^2,
+// 512^2 and 1024^2). Masked grids of at least 1024^2 cells run the stored-form TMA march
+// (configuration 11), smaller ones the tile kernel.
 int default_stage_config_mixed(long long cells, bool mask)
 {
-    return cells >= 1024LL * 1024 ? (mask ? 11 : 17) : 0;
+    if (mask) {
+        return cells >= 1024LL * 1024 ? 11 : 0;
+    }
+    return cells >= 768LL * 768 ? 17 : 18;
 }
 
 TileConfigInfo stage_config_info_mixed(int c) { return kInfo[c < 0 || c >= kCount ? 0 : c]; }
@@ -87,6 +95,8 @@ StageKernels select_stage_mixed(int limiter, bool nonideal, bool mask, int confi
         return select_unmasked<PolicyMixed, Cfg16>(limiter, nonideal, mask);
     case 17:
         return select_full<PolicyMixed, Cfg17>(limiter, nonideal, mask);
+    case 18:
+        return select_unmasked<PolicyMixed, Cfg18>(limiter, nonideal, mask);
     default:
         return select_full<PolicyMixed, Cfg0>(limiter, nonideal, mask);
     }

@@ -1,6 +1,6 @@
 // Warp-synchronous strip-march stage kernel (ideal or non-ideal GLM-MHD, no solid mask).
 //
-// Each warp owns a strip of kMarchOwned = 28 columns and a segment of LY rows. Lane l holds
+// Each warp owns a strip of kMarchOwned = 28 columns and a segment of Args::rows rows. Lane l holds
 // column x0 - 2 + l (lanes 0, 1 and 30, 31 are the x halo) and the warp marches up the segment
 // one row at a time, so the whole stencil lives in registers:
 //   * the primitives of rows j and j+1, the y slope of row j and the y flux G(j-1/2) are carried
@@ -16,7 +16,7 @@
 // formed from rows y, y + 1, y + 2 and the x neighbours by shuffles, and both face fluxes get the
 // Ohm's-law correction from face-averaged J and B, as in the tile kernel.
 //
-// A block is NW warps side by side (NW * 28 columns x LY rows), so the host's tile grid
+// A block is NW warps side by side (NW * 28 columns x rows), so the host's tile grid
 // arithmetic is the same as for the tile kernel.
 #pragma once
 
@@ -61,7 +61,7 @@ __device__ __forceinline__ void march_nonideal_y(const T (&Jb)[3], const T (&Wb)
                                Wa[5], Wa[6], Wa[7], ni, G);
 }
 
-template <class Policy, int L, int STAGE, int LY, bool NI = false>
+template <class Policy, int L, int STAGE, bool NI = false>
 __device__ __forceinline__ double march_strip(const typename Policy::Args& a, int x0, int y0,
                                               int lane)
 {
@@ -82,7 +82,7 @@ __device__ __forceinline__ double march_strip(const typename Policy::Args& a, in
     const int gx = x0 - 2 + lane;
     const int sx = map_index(gx, g.nx, g.bc_x);
     const bool own = lane >= 2 && lane < 2 + kMarchOwned && gx < g.nx;
-    const int y1 = min(y0 + LY, g.ny);
+    const int y1 = min(y0 + a.rows, g.ny);
 
     auto load = [&](int y, Raw& r) { Policy::load_raw(a, g, sx, map_index(y, g.ny, g.bc_y), r); };
     auto prim = [&](int y, const Raw& r, T (&w)[9]) {
@@ -194,7 +194,7 @@ __device__ __forceinline__ double march_strip(const typename Policy::Args& a, in
     return smax;
 }
 
-template <class Policy, int L, int STAGE, int LY, int NW, int MINB, bool NI = false>
+template <class Policy, int L, int STAGE, int NW, int MINB, bool NI = false>
 __global__ void __launch_bounds__(NW * 32, MINB) march_kernel(const typename Policy::Args a)
 {
     if (a.ctrl->finished != 0) {
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) march_kernel(const typename Pol
     const int x0 = strip * kMarchOwned;
     double smax = 0.0;
     if (x0 < a.geom.nx) { // warp-uniform
-        smax = march_strip<Policy, L, STAGE, LY, NI>(a, x0, static_cast<int>(blockIdx.y) * LY, lane);
+        smax = march_strip<Policy, L, STAGE, NI>(a, x0, static_cast<int>(blockIdx.y) * a.rows, lane);
     }
     if constexpr (STAGE == 2) {
         reduce_signal_speed_and_finish(smax, a.ctrl, a.k, gridDim.x * gridDim.y, true);
@@ -213,11 +213,11 @@ __global__ void __launch_bounds__(NW * 32, MINB) march_kernel(const typename Pol
 }
 
 // Persistent strip-march form over a block work-list of many independent solves (each item:
-// solve index, block index; a block is NW strips of 28 columns by LY rows; Desc is any
+// solve index, block index; a block is NW strips of 28 columns by Args::rows rows; Desc is any
 // descriptor with stage[2], tiles_x and ntiles). Every CTA walks the
 // list with a grid stride, like batch_stage_kernel in stage_kernel.cuh; a solve's signal-speed
 // reduction completes when its last block arrives and that block advances the solve's clock.
-template <class Policy, int L, bool NI, int STAGE, int LY, int NW, int MINB,
+template <class Policy, int L, bool NI, int STAGE, int NW, int MINB,
           class Desc = BatchSolve<Policy>>
 __global__ void __launch_bounds__(NW * 32, MINB) batch_march_kernel(const Desc* solves,
                                                                      const int2* __restrict__ work,
@@ -246,10 +246,10 @@ __global__ void __launch_bounds__(NW * 32, MINB) batch_march_kernel(const Desc* 
             continue;
         }
         const int x0 = ((it.y % s_tiles_x) * NW + warp) * kMarchOwned;
-        const int y0 = (it.y / s_tiles_x) * LY;
+        const int y0 = (it.y / s_tiles_x) * sa.rows;
         double smax = 0.0;
         if (x0 < sa.geom.nx) { // warp-uniform
-            smax = march_strip<Policy, L, STAGE, LY, NI>(sa, x0, y0, lane);
+            smax = march_strip<Policy, L, STAGE, NI>(sa, x0, y0, lane);
         }
         if constexpr (STAGE == 2) {
             reduce_signal_speed_and_finish(smax, sa.ctrl, sa.k, static_cast<unsigned>(s_ntiles),

@@ -87,7 +87,7 @@ static_assert(fits_16_blocks(march_tma_smem_bytes<1, 1>(1)) &&
                   fits_16_blocks(march_tma_smem_bytes<2, 0, 4, 2>(1)),
               "a one-warp FP32-mixed strip-march layout no longer fits 16 blocks per SM");
 
-template <int L, int STAGE, int LY, bool HF, int ST, bool NI, bool MASK = false,
+template <int L, int STAGE, bool HF, int ST, bool NI, bool MASK = false,
           class Policy = PolicyMixed>
 __device__ __forceinline__ double march_tma_strip(const typename Policy::Args& a,
                                                   const MarchTmaMaps& m,
@@ -115,8 +115,7 @@ __device__ __forceinline__ double march_tma_strip(const typename Policy::Args& a
     const int sx = map_index(gx, g.nx, g.bc_x);
     const bool in_x = gx >= 0 && gx < g.nx;
     const bool own = lane >= 2 && lane < 2 + kMarchOwned && gx < g.nx;
-    const int y1 = min(y0 + LY, g.ny);
-    const int nrows = y1 - y0;
+    const int nrows = min(a.rows, g.ny - y0);
 
     const T* halo_f = reinterpret_cast<const T*>(wbase);
     const T* own_f = reinterpret_cast<const T*>(wbase + 2 * Lay::kHaloSlot);
@@ -587,7 +586,7 @@ __device__ __forceinline__ double march_tma_strip(const typename Policy::Args& a
     return smax;
 }
 
-template <int L, int STAGE, int LY, int NW, int MINB, bool HF, int ST, bool NI, bool MASK = false,
+template <int L, int STAGE, int NW, int MINB, bool HF, int ST, bool NI, bool MASK = false,
           class Policy = PolicyMixed>
 __global__ void __launch_bounds__(NW * 32, MINB) march_tma_kernel(const typename Policy::Args a,
                                                                    const __grid_constant__ MarchTmaMaps m)
@@ -605,8 +604,8 @@ __global__ void __launch_bounds__(NW * 32, MINB) march_tma_kernel(const typename
     bool failed = false;
     if (x0 < a.geom.nx) { // warp-uniform
         static_assert(!MASK || ST == 0, "masked strips store through the lanes");
-        smax = march_tma_strip<L, STAGE, LY, HF, ST, NI, MASK, Policy>(
-            a, m, x0, static_cast<int>(blockIdx.y) * LY, lane,
+        smax = march_tma_strip<L, STAGE, HF, ST, NI, MASK, Policy>(
+            a, m, x0, static_cast<int>(blockIdx.y) * a.rows, lane,
             base + warp * MarchTmaLayout<STAGE, ST, sizeof(typename Policy::T),
                                          Policy::kLayout>::kWarpBytes,
             failed);
@@ -633,7 +632,7 @@ struct BatchSolveTma {
 // index, block index), as batch_march_kernel; the tensor maps come from the descriptor array in
 // global memory (lane 0 acquires them before its copies). A warp whose copies timed out processes
 // no further items: the solves of the items it would have run report kStatusWaitTimeout too.
-template <int L, bool NI, int STAGE, int LY, int NW, int MINB, bool HF, int ST>
+template <int L, bool NI, int STAGE, int NW, int MINB, bool HF, int ST>
 __global__ void __launch_bounds__(NW * 32, MINB) batch_march_tma_kernel(
     const BatchSolveTma* solves, const int2* __restrict__ work, int nwork)
 {
@@ -665,7 +664,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) batch_march_tma_kernel(
         }
         const MarchTmaMaps& m = solves[it.x].maps[STAGE - 1];
         const int x0 = ((it.y % s_tiles_x) * NW + warp) * kMarchOwned;
-        const int y0 = (it.y / s_tiles_x) * LY;
+        const int y0 = (it.y / s_tiles_x) * sa.rows;
         double smax = 0.0;
         if (x0 < sa.geom.nx && failed) { // warp-uniform
             // this warp's barriers are unusable after a timed-out wait, so it cannot advance the
@@ -680,7 +679,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) batch_march_tma_kernel(
                 tensormap_acquire(&m.out_own);
             }
             __syncwarp();
-            smax = march_tma_strip<L, STAGE, LY, HF, ST, NI>(sa, m, x0, y0, lane, wbase, failed);
+            smax = march_tma_strip<L, STAGE, HF, ST, NI>(sa, m, x0, y0, lane, wbase, failed);
         }
         if constexpr (STAGE == 2) {
             reduce_signal_speed_and_finish(smax, sa.ctrl, sa.k, static_cast<unsigned>(s_ntiles),
@@ -692,7 +691,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) batch_march_tma_kernel(
 // The batch kernel of the increment form: as batch_march_tma_kernel, with each solve's
 // arguments and tensor maps taken for the state-buffer parity of its step counter (read before
 // the stage; it only changes when the solve's stage-2 reduction completes).
-template <int L, bool NI, int STAGE, int LY, int NW, int MINB, bool HF>
+template <int L, bool NI, int STAGE, int NW, int MINB, bool HF>
 __global__ void __launch_bounds__(NW * 32, MINB) batch_march_delta_kernel(
     const BatchSolveTma* solves, const int2* __restrict__ work, int nwork)
 {
@@ -726,7 +725,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) batch_march_delta_kernel(
         }
         const MarchTmaMaps& m = solves[it.x].dmaps[s_q][STAGE - 1];
         const int x0 = ((it.y % s_tiles_x) * NW + warp) * kMarchOwned;
-        const int y0 = (it.y / s_tiles_x) * LY;
+        const int y0 = (it.y / s_tiles_x) * sa.rows;
         double smax = 0.0;
         if (x0 < sa.geom.nx && failed) { // warp-uniform: as in batch_march_tma_kernel
             if (lane == 0) {
@@ -742,7 +741,7 @@ __global__ void __launch_bounds__(NW * 32, MINB) batch_march_delta_kernel(
                 }
             }
             __syncwarp();
-            smax = march_tma_strip<L, STAGE, LY, HF, 0, NI, false, PolicyDelta<STAGE, 2>>(
+            smax = march_tma_strip<L, STAGE, HF, 0, NI, false, PolicyDelta<STAGE, 2>>(
                 sa, m, x0, y0, lane, wbase, failed);
         }
         if constexpr (STAGE == 2) {

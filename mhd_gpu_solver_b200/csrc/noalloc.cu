@@ -15,6 +15,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstdio>
@@ -175,7 +176,11 @@ int mhdb_solve_steps_noalloc_f64(const mhdb_grid* grid, int bc_x, int bc_y,
                (params->hall && params->eta_hall != 0.0) ||
                (params->ambipolar && params->eta_ambipolar != 0.0);
 
-    const StageKernels sk = select_stage_f64(params->limiter, k.ni_any != 0, false, 0);
+    // The caller's dense planes have any row pitch and base alignment, so where a handle's solve of
+    // this size marches with bulk copies this one takes the register march (configuration 8).
+    const int dflt = default_stage_config_f64(static_cast<long long>(cells), false, k.ni_any != 0);
+    const int cfg = dflt == 7 ? 8 : dflt;
+    const StageKernels sk = select_stage_f64(params->limiter, k.ni_any != 0, false, cfg);
     if (sk.threads == 0) {
         return fail(MHDB_INVALID_ARGUMENT, "no stage kernel for this configuration");
     }
@@ -218,12 +223,17 @@ int mhdb_solve_steps_noalloc_f64(const mhdb_grid* grid, int bc_x, int bc_y,
     const int init_blocks =
         static_cast<int>(std::min<long long>((ncell + 255) / 256, 148LL * 8));
     noalloc_cfl_init<256><<<init_blocks, 256, 0, s>>>(u_out, g, k, ctrl);
-    const StageArgsF64 a1{u_out, ustar, nullptr, ctrl, g, k, 1};
-    const StageArgsF64 a2{ustar, u_out, nullptr, ctrl, g, k, 1};
-    const dim3 grid2((grid->nx + sk.tile_x - 1) / sk.tile_x, (grid->ny + sk.tile_y - 1) / sk.tile_y);
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int rows = sk.segments ? segment_rows(grid->nx, grid->ny, sk.tile_x, sk.tile_y,
+                                                sms * sk.min_blocks)
+                                 : sk.tile_y;
+    const StageArgsF64 a1{u_out, ustar, nullptr, ctrl, g, k, 1, rows};
+    const StageArgsF64 a2{ustar, u_out, nullptr, ctrl, g, k, 1, rows};
+    const dim3 blocks((grid->nx + sk.tile_x - 1) / sk.tile_x, (grid->ny + rows - 1) / rows);
     for (int i = 0; i < nsteps; ++i) {
-        sk.f64_stage1<<<grid2, sk.threads, sk.smem, s>>>(a1);
-        sk.f64_stage2<<<grid2, sk.threads, sk.smem, s>>>(a2);
+        sk.f64_stage1<<<blocks, sk.threads, sk.smem, s>>>(a1);
+        sk.f64_stage2<<<blocks, sk.threads, sk.smem, s>>>(a2);
     }
     e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -86,13 +86,18 @@ __device__ __forceinline__ int map_index(int x, int n, int bc)
 __device__ __forceinline__ void finish_step(Ctrl* ctrl, const Consts& k, bool advance)
 {
     const double c_h = __longlong_as_double(static_cast<long long>(atomicExch(&ctrl->ch_bits, 0ull)));
+    double t = ctrl->t;
+    int steps = ctrl->steps;
+    const double dt_done = ctrl->dt, t_end = ctrl->t_end;
+    const int max_steps = ctrl->max_steps, status = ctrl->status;
     ctrl->arrived = 0u;
     if (advance) {
-        ctrl->t += ctrl->dt;
-        ctrl->steps += 1;
+        t += dt_done;
+        steps += 1;
+        ctrl->t = t;
+        ctrl->steps = steps;
     }
-    if (!(ctrl->t < ctrl->t_end) || ctrl->steps >= ctrl->max_steps ||
-        (ctrl->status & kStatusWaitTimeout) != 0) {
+    if (!(t < t_end) || steps >= max_steps || (status & kStatusWaitTimeout) != 0) {
         ctrl->finished = 1;
         return;
     }
@@ -101,9 +106,9 @@ __device__ __forceinline__ void finish_step(Ctrl* ctrl, const Consts& k, bool ad
     if (k.eta_max > 0.0) {
         dt = vmin(dt, k.dt_diff);
     }
-    dt = vmin(dt, ctrl->t_end - ctrl->t);
+    dt = vmin(dt, t_end - t);
     if (!(dt > 0.0) || isinf(dt)) {
-        ctrl->status |= kStatusBadDt;
+        ctrl->status = status | kStatusBadDt;
         ctrl->finished = 1;
         return;
     }

@@ -209,6 +209,7 @@ struct mhdb_solver {
     mhdb_grid grid{};
     int precision = MHDB_FP64;
     int device = 0;
+    int sms = 148;
     std::string name;
     std::string last_error;
     cudaStream_t stream = nullptr;
@@ -371,6 +372,42 @@ struct StepPlan {
     Consts k{};
 };
 
+} // namespace
+
+namespace mhdb {
+
+// Rows of a strip march's segments: the split of the grid's rows whose blocks cost least, for
+// `slots` blocks resident on the GPU. A block marches its rows one after the other (a row of a lone
+// FP32-mixed stage takes about 1.3 us, of an FP64 one 1.7 us), so few long segments leave a small
+// grid waiting on that chain with most of the GPU idle, and many short ones pay a prologue of
+// about 1.3 rows each. With w = blocks / slots, a row takes 1 + w of a lone block's time up to one
+// full wave (measured from w = 0.1 to 1 in both precision forms); beyond, 2 w and the idle part of
+// the last wave, which costs less the more waves there are. Measured per step, 32-row segments ->
+// this rule: FP32-mixed 512^2 100 -> 39 us, 1024^2 127 -> 100 us; FP64 512^2 134 -> 53 us,
+// 1448^2 342 -> 300 us; from 2048^2 up within 3 % of 32 rows.
+int segment_rows(int nx, int ny, int tile_x, int most, int slots)
+{
+    const int strips = (nx + tile_x - 1) / tile_x;
+    int best = most;
+    double least = INFINITY;
+    for (int rows = std::min(most, ny); rows >= 1; --rows) {
+        const int segments = (ny + rows - 1) / rows;
+        const double w = static_cast<double>(strips) * segments / slots;
+        const double idle = std::ceil(w) - w; // of the last wave
+        const double tail = idle * std::max(0.0, 1.05 - 0.25 * std::floor(w));
+        const double cost = (rows + 1.3) * (w <= 1.0 ? 1.0 + w : 2.0 * w + tail);
+        if (cost < least) {
+            least = cost;
+            best = rows;
+        }
+    }
+    return best;
+}
+
+} // namespace mhdb
+
+namespace {
+
 StepPlan make_plan(mhdb_solver* h, const mhdb_params* p)
 {
     StepPlan s;
@@ -383,7 +420,7 @@ StepPlan make_plan(mhdb_solver* h, const mhdb_params* p)
     // solve the chosen configuration does not serve (e.g. a masked solve after an autotuner
     // choice made on unmasked grids) uses the default configuration of its size, else 0.
     const long long cells = static_cast<long long>(h->grid.nx) * h->grid.ny;
-    const int dflt = h->precision == MHDB_FP64 ? default_stage_config_f64(cells, h->has_mask)
+    const int dflt = h->precision == MHDB_FP64 ? default_stage_config_f64(cells, h->has_mask, ni)
                                                : default_stage_config_mixed(cells, h->has_mask);
     auto serves = [&](int c) {
         return c == 0 || (h->precision == MHDB_FP64
@@ -459,7 +496,14 @@ StepPlan make_plan(mhdb_solver* h, const mhdb_params* p)
     if (sk.threads == 0) {
         throw ApiError{MHDB_INVALID_ARGUMENT, "no stage kernel for this configuration"};
     }
-    s.grid = dim3((h->grid.nx + sk.tile_x - 1) / sk.tile_x, (h->grid.ny + sk.tile_y - 1) / sk.tile_y);
+    const int rows = sk.segments ? segment_rows(h->grid.nx, h->grid.ny, sk.tile_x, sk.tile_y,
+                                          h->sms * sk.min_blocks)
+                           : sk.tile_y;
+    s.a1.rows = s.a2.rows = s.b1.rows = s.b2.rows = rows;
+    for (int q = 0; q < 2; ++q) {
+        s.c1[q].rows = s.c2[q].rows = rows;
+    }
+    s.grid = dim3((h->grid.nx + sk.tile_x - 1) / sk.tile_x, (h->grid.ny + rows - 1) / rows);
     s.block = dim3(sk.threads);
     s.smem = sk.smem;
     s.smem2 = sk.smem2;
@@ -854,6 +898,7 @@ int mhdb_create(const mhdb_grid* grid, int precision, mhdb_solver** out)
         cudaDeviceProp prop{};
         MHDB_CHECK(cudaGetDeviceProperties(&prop, h->device));
         h->name = std::string("CUDA: ") + prop.name;
+        h->sms = prop.multiProcessorCount;
         MHDB_CHECK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
         h->nxt = grid->nx + 2 * grid->ng;
         h->nyt = grid->ny + 2 * grid->ng;

@@ -31,6 +31,7 @@ struct StageArgsDelta {
     Geometry geom;
     Consts k;
     int walls;
+    int rows;            // rows of a warp's segment (TMA strip marches)
 };
 
 // LAYOUT: MarchTmaLayout kind of the TMA strip march (1: own cells' delta through the own

@@ -30,6 +30,8 @@ struct StageKernels {
     StageFnDeltaTma dx_tma1 = nullptr, dx_tma2 = nullptr; // FP32-mixed increment form
     int tile_x = 0, tile_y = 0, threads = 0; // threads == 0: no such configuration
     size_t smem = 0, smem2 = 0;               // dynamic shared memory per block, stage 1 and 2
+    bool segments = false; // tile_y is the most rows of a segment; the plan picks them
+    int min_blocks = 0;    // blocks resident per SM (segments)
     int halo_w = kTmaHaloW, own_w = kTmaOwnW; // TMA box widths of the increment form's maps
 };
 
@@ -51,8 +53,11 @@ struct TileConfigInfo {
 // Number of tile configurations compiled per precision form, and their shapes.
 int stage_config_count_f64();
 int stage_config_count_mixed();
+// Rows of the segments a grid is split into by a strip march with blocks of tile_x columns and at
+// most `most` rows, of which `slots` are resident on the GPU (solver.cu).
+int segment_rows(int nx, int ny, int tile_x, int most, int slots);
 // Configuration used when none is chosen (mhdb_set_tile_config(h, -1), the default).
-int default_stage_config_f64(long long cells, bool mask);
+int default_stage_config_f64(long long cells, bool mask, bool nonideal);
 int default_stage_config_mixed(long long cells, bool mask);
 TileConfigInfo stage_config_info_f64(int config);
 TileConfigInfo stage_config_info_mixed(int config);
