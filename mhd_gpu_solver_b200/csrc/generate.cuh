@@ -16,7 +16,7 @@
 namespace mhdb {
 
 constexpr int kGenThreads = 256;
-constexpr int kGenBlocks = 296;
+constexpr int kGenBlocks = 1184; // 8 x 148 SMs
 
 struct GenSpec {
     int kind; // 0 Fourier, 1 four quadrants
@@ -28,6 +28,15 @@ struct GenSpec {
 
 // Raw Fourier fields into the scratch planes: 0 f1, 1 vx, 2 vy, 4 f2, 5 bx, 6 by (unscaled),
 // and per-block partial sums of vx^2+vy^2, bx^2+by^2, f1^2, f2^2.
+//
+// A block takes 256 cells of one row at a time. The sum over ky is the same for all of them, so it
+// is done once per item into shared memory, D_q[kx] = sum_ky C_q[ky][kx] exp(i 2 pi ky uy) (and the
+// same of i w_y C for A_z's y derivative), and each cell adds KX terms Re(D_q[kx] exp(i 2 pi kx ux))
+// with KX sincospi in place of 2 KX KY: FP64-bound, 141 -> 17 us for the mean solve of a batch of
+// sides 64-1024 (1.2e5 cells, kmax 8). kx and ky go in chunks, so any kmax fits.
+constexpr int kGenChunk = 32;
+constexpr int kGenFields = 6; // vx, vy, dA/dy, A (for dA/dx), f1, f2
+
 static __global__ void __launch_bounds__(kGenThreads) gen_fourier_raw(const double2* __restrict__ coef,
                                                               GenSpec s, Geometry g,
                                                               double* __restrict__ scratch,
@@ -35,48 +44,83 @@ static __global__ void __launch_bounds__(kGenThreads) gen_fourier_raw(const doub
 {
     const int K = s.kmax;
     const int KX = K + 1, KY = 2 * K + 1, NC = KX * KY;
-    const double lx = s.x_max - s.x_min, ly = s.y_max - s.y_min;
+    const double wx = 2.0 * M_PI / (s.x_max - s.x_min), wy = 2.0 * M_PI / (s.y_max - s.y_min);
+    __shared__ double2 ey[kGenChunk];
+    __shared__ double2 D[kGenChunk][kGenFields];
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    const long long n = static_cast<long long>(g.nx) * g.ny;
-    for (long long c = blockIdx.x * static_cast<long long>(kGenThreads) + threadIdx.x; c < n;
-         c += static_cast<long long>(gridDim.x) * kGenThreads) {
-        const int x = static_cast<int>(c % g.nx), y = static_cast<int>(c / g.nx);
+    const int tiles_x = (g.nx + kGenThreads - 1) / kGenThreads;
+    const long long items = static_cast<long long>(tiles_x) * g.ny;
+    for (long long it = blockIdx.x; it < items; it += gridDim.x) {
+        const int y = static_cast<int>(it / tiles_x);
+        const int x = static_cast<int>(it % tiles_x) * kGenThreads + static_cast<int>(threadIdx.x);
         const double ux = (x + 0.5) / g.nx, uy = (y + 0.5) / g.ny; // (x - x_min)/lx
-        double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0}; // vx, vy, bx, by, and (f1, f2 below)
-        double f1 = 0.0, f2 = 0.0;
-        for (int iy = 0; iy < KY; ++iy) {
-            const int ky = iy - K;
-            double sy, cy;
-            sincospi(2.0 * ky * uy, &sy, &cy);
-            for (int kx = 0; kx <= K; ++kx) {
-                double sx, cx;
-                sincospi(2.0 * kx * ux, &sx, &cx);
-                // e = exp(i 2 pi (kx ux + ky uy))
-                const double er = cx * cy - sx * sy, ei = sx * cy + cx * sy;
-                const int m = iy * KX + kx;
-                const double2 cvx = coef[0 * NC + m], cvy = coef[1 * NC + m];
-                const double2 caz = coef[2 * NC + m], cf1 = coef[3 * NC + m], cf2 = coef[4 * NC + m];
-                v[0] += cvx.x * er - cvx.y * ei;
-                v[1] += cvy.x * er - cvy.y * ei;
-                // Re(C (i w) e) = -w Im(C e)
-                const double im_az = caz.x * ei + caz.y * er;
-                v[2] += -(2.0 * M_PI / ly) * ky * im_az;  // bx = dA/dy
-                v[3] += (2.0 * M_PI / lx) * kx * im_az;   // by = -dA/dx
-                f1 += cf1.x * er - cf1.y * ei;
-                f2 += cf2.x * er - cf2.y * ei;
+        double v[kGenFields] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        for (int kx0 = 0; kx0 < KX; kx0 += kGenChunk) {
+            const int nkx = min(kGenChunk, KX - kx0);
+            // D of this chunk: one (kx, field) per thread
+            const int dk = threadIdx.x % kGenChunk, dq = threadIdx.x / kGenChunk;
+            const bool dwork = dq < kGenFields && dk < nkx;
+            double dr = 0.0, di = 0.0;
+            for (int iy0 = 0; iy0 < KY; iy0 += kGenChunk) {
+                const int nky = min(kGenChunk, KY - iy0);
+                __syncthreads(); // the previous chunk's ey and D have been read
+                if (static_cast<int>(threadIdx.x) < nky) {
+                    double sy, cy;
+                    sincospi(2.0 * (iy0 + static_cast<int>(threadIdx.x) - K) * uy, &sy, &cy);
+                    ey[threadIdx.x] = make_double2(cy, sy);
+                }
+                __syncthreads();
+                if (dwork) {
+                    // spectra: 0 vx, 1 vy, 2 A_z, 3 f1, 4 f2
+                    const int spec = dq < 2 ? dq : (dq < 4 ? 2 : dq - 1);
+                    for (int j = 0; j < nky; ++j) {
+                        const double2 c = coef[spec * NC + (iy0 + j) * KX + kx0 + dk];
+                        const double er = ey[j].x, ei = ey[j].y;
+                        const double pr = c.x * er - c.y * ei, pi = c.x * ei + c.y * er;
+                        if (dq == 2) { // times i w_y ky
+                            const double w = wy * (iy0 + j - K);
+                            dr -= w * pi;
+                            di += w * pr;
+                        } else {
+                            dr += pr;
+                            di += pi;
+                        }
+                    }
+                }
+            }
+            if (dwork) {
+                if (dq == 3) { // times -i w_x kx: By = -dA/dx
+                    const double w = wx * (kx0 + dk);
+                    D[dk][dq] = make_double2(w * di, -w * dr);
+                } else {
+                    D[dk][dq] = make_double2(dr, di);
+                }
+            }
+            __syncthreads();
+            if (x < g.nx) {
+                for (int k = 0; k < nkx; ++k) {
+                    double sx, cx;
+                    sincospi(2.0 * (kx0 + k) * ux, &sx, &cx);
+#pragma unroll
+                    for (int q = 0; q < kGenFields; ++q) {
+                        v[q] += D[k][q].x * cx - D[k][q].y * sx;
+                    }
+                }
             }
         }
-        const size_t o = static_cast<size_t>(y) * g.pitch + x;
-        scratch[0 * g.plane + o] = f1;
-        scratch[1 * g.plane + o] = v[0];
-        scratch[2 * g.plane + o] = v[1];
-        scratch[4 * g.plane + o] = f2;
-        scratch[5 * g.plane + o] = v[2];
-        scratch[6 * g.plane + o] = v[3];
-        acc[0] += v[0] * v[0] + v[1] * v[1];
-        acc[1] += v[2] * v[2] + v[3] * v[3];
-        acc[2] += f1 * f1;
-        acc[3] += f2 * f2;
+        if (x < g.nx) {
+            const size_t o = static_cast<size_t>(y) * g.pitch + x;
+            scratch[0 * g.plane + o] = v[4];
+            scratch[1 * g.plane + o] = v[0];
+            scratch[2 * g.plane + o] = v[1];
+            scratch[4 * g.plane + o] = v[5];
+            scratch[5 * g.plane + o] = v[2];
+            scratch[6 * g.plane + o] = v[3];
+            acc[0] += v[0] * v[0] + v[1] * v[1];
+            acc[1] += v[2] * v[2] + v[3] * v[3];
+            acc[2] += v[4] * v[4];
+            acc[3] += v[5] * v[5];
+        }
     }
     __shared__ double sh[4][kGenThreads];
     for (int q = 0; q < 4; ++q) {
@@ -102,15 +146,24 @@ __global__ void __launch_bounds__(kGenThreads) gen_finish(Store store, GenSpec s
                                                          const double* __restrict__ partial,
                                                          int nblocks)
 {
-    // scale factors from the block partials (summed in block order by every thread)
-    double sum[4] = {0.0, 0.0, 0.0, 0.0};
-    if (s.kind == 0) {
-        for (int b = 0; b < nblocks; ++b) {
-            for (int q = 0; q < 4; ++q) {
-                sum[q] += partial[q * nblocks + b];
+    // scale factors from the block partials: warp q sums the q-th, in a fixed order
+    __shared__ double sum[4];
+    if (threadIdx.x < 128) {
+        const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double v = 0.0;
+        if (s.kind == 0) {
+            for (int b = lane; b < nblocks; b += 32) {
+                v += partial[q * nblocks + b];
             }
         }
+        for (int o = 16; o > 0; o >>= 1) {
+            v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
+        if (lane == 0) {
+            sum[q] = v;
+        }
     }
+    __syncthreads();
     const double ncell = static_cast<double>(g.nx) * g.ny;
     const double vs = 1.0 / sqrt(sum[0] / ncell), bs = 1.0 / sqrt(sum[1] / ncell);
     const double f1s = sqrt(sum[2] / ncell), f2s = sqrt(sum[3] / ncell);
@@ -175,18 +228,25 @@ struct StoreMx {
 namespace mhdb {
 
 // Host side: generate an initial state into `store` using `scratch` (9 double planes of the
-// solve's geometry, e.g. its stage buffer). Allocates two small stream-ordered buffers (the
-// spectra and the rms partials) and frees them on the stream.
+// solve's geometry, e.g. its stage buffer). The spectra and the rms partials go into scratch's last
+// two planes, which the raw fields leave free (stream-ordered allocations in their place made
+// admitting a solve wait 2-6 ms for the driver: the default pool gives its memory back at every
+// synchronisation); only a grid too small to hold them allocates two stream-ordered buffers.
 template <class Store>
 inline cudaError_t launch_generate(cudaStream_t st, const GenSpec& spec, const double* coef_host,
                                    const Geometry& g, double* scratch, Store store)
 {
-    double2* coef = nullptr;
-    double* partial = nullptr;
-    cudaError_t e = cudaSuccess;
+    if (spec.kind != 0) {
+        gen_finish<<<kGenBlocks, kGenThreads, 0, st>>>(store, spec, g, scratch, nullptr, 0);
+        return cudaGetLastError();
+    }
     const int nblocks = kGenBlocks;
-    if (spec.kind == 0) {
-        const size_t nc = static_cast<size_t>(5) * (2 * spec.kmax + 1) * (spec.kmax + 1);
+    const size_t nc = static_cast<size_t>(5) * (2 * spec.kmax + 1) * (spec.kmax + 1);
+    const bool fits = 2 * nc + 4 * nblocks <= 2 * g.plane;
+    double2* coef = reinterpret_cast<double2*>(scratch + 7 * g.plane); // plane: a multiple of 32
+    double* partial = scratch + 7 * g.plane + 2 * nc;
+    cudaError_t e = cudaSuccess;
+    if (!fits) {
         if ((e = cudaMallocAsync(reinterpret_cast<void**>(&coef), nc * sizeof(double2), st)) != cudaSuccess) {
             return e;
         }
@@ -194,18 +254,18 @@ inline cudaError_t launch_generate(cudaStream_t st, const GenSpec& spec, const d
             cudaFreeAsync(coef, st);
             return e;
         }
-        e = cudaMemcpyAsync(coef, coef_host, nc * sizeof(double2), cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) {
-            gen_fourier_raw<<<nblocks, kGenThreads, 0, st>>>(coef, spec, g, scratch, partial);
-            gen_finish<<<nblocks, kGenThreads, 0, st>>>(store, spec, g, scratch, partial, nblocks);
-            e = cudaGetLastError();
-        }
+    }
+    e = cudaMemcpyAsync(coef, coef_host, nc * sizeof(double2), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) {
+        gen_fourier_raw<<<nblocks, kGenThreads, 0, st>>>(coef, spec, g, scratch, partial);
+        gen_finish<<<nblocks, kGenThreads, 0, st>>>(store, spec, g, scratch, partial, nblocks);
+        e = cudaGetLastError();
+    }
+    if (!fits) {
         cudaFreeAsync(coef, st);
         cudaFreeAsync(partial, st);
-        return e;
     }
-    gen_finish<<<nblocks, kGenThreads, 0, st>>>(store, spec, g, scratch, nullptr, 0);
-    return cudaGetLastError();
+    return e;
 }
 
 } // namespace mhdb
