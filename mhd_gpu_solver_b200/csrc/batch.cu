@@ -798,10 +798,8 @@ void add_solve(mhdb_batch* b, const mhdb_grid* grid, const mhdb_params* params, 
             cudaFreeAsync(s.Us, b->stream);
             check(e3, "cudaMallocFromPoolAsync(staging)");
         }
-        for (int c = 0; c < 9; ++c) {
-            check(cudaMemcpyAsync(stg + c * n_tot, comps[c], n_tot * sizeof(double),
-                                  cudaMemcpyHostToDevice, b->stream), "cudaMemcpyAsync(state)");
-        }
+        check(copy_planes(stg, comps, n_tot, cudaMemcpyHostToDevice, b->stream),
+              "cudaMemcpyAsync(state)");
         if (b->precision == MHDB_FP64) {
             batch_unpack_f64<<<blocks_for(n, 256), 256, 0, b->stream>>>(stg, static_cast<double*>(s.U), s.geom, grid->ng, nxt, n_tot);
         } else {
@@ -1105,10 +1103,8 @@ int mhdb_batch_download(mhdb_batch* b, int id, double* const comps[9], size_t n_
         }
         ++b->launches;
         check(cudaGetLastError(), "batch pack launch");
-        for (int c = 0; c < 9; ++c) {
-            check(cudaMemcpyAsync(comps[c], stg + c * n_tot, n_tot * sizeof(double),
-                                  cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync(download)");
-        }
+        check(copy_planes(stg, comps, n_tot, cudaMemcpyDeviceToHost, st),
+              "cudaMemcpyAsync(download)");
         check(cudaFreeAsync(stg, st), "cudaFreeAsync(staging)");
         check(cudaStreamSynchronize(st), "cudaStreamSynchronize");
     });

@@ -4,6 +4,8 @@
 #include <cstddef>
 #include <cstdint>
 
+#include <cuda_runtime.h>
+
 #include "physics.cuh"
 
 namespace mhdb {
@@ -64,6 +66,42 @@ struct Ctrl {
     // launches finish_step_kernel.
     int defer;
 };
+
+// Copy nine host planes of n doubles to or from nine consecutive device planes: one copy where the
+// host planes follow one another too (an array of shape (9, ny, nx)), as every copy costs a launch
+// of about 5 us and starts the link anew; plane by plane otherwise, or where the driver refuses a
+// copy across host buffers that only happen to be neighbours.
+template <class Host>
+inline cudaError_t copy_planes(double* device, Host* const host[9], size_t n, cudaMemcpyKind kind,
+                               cudaStream_t stream)
+{
+    const bool to_device = kind == cudaMemcpyHostToDevice;
+    const size_t bytes = n * sizeof(double);
+    auto copy = [&](int c, size_t b) {
+        void* h = const_cast<double*>(host[c]);
+        double* d = device + static_cast<size_t>(c) * n;
+        return cudaMemcpyAsync(to_device ? static_cast<void*>(d) : h, to_device ? h : d, b, kind,
+                               stream);
+    };
+    bool consecutive = true;
+    for (int c = 1; c < 9; ++c) {
+        consecutive = consecutive && host[c] == host[0] + static_cast<size_t>(c) * n;
+    }
+    if (consecutive) {
+        const cudaError_t e = copy(0, 9 * bytes);
+        if (e != cudaErrorInvalidValue) {
+            return e;
+        }
+        cudaGetLastError(); // refused before anything was copied
+    }
+    for (int c = 0; c < 9; ++c) {
+        const cudaError_t e = copy(c, bytes);
+        if (e != cudaSuccess) {
+            return e;
+        }
+    }
+    return cudaSuccess;
+}
 
 // Boundary rule as an index map onto the interior (include/boundary_conditions/
 // boundary_conditions.hpp:26-88): periodic wraps modulo n (valid for any offset, also when

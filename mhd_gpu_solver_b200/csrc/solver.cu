@@ -720,6 +720,16 @@ int steps_to_queue(const Ctrl& c)
     return n;
 }
 
+template <class P>
+void require_components(P* const comps[9])
+{
+    for (int c = 0; c < 9; ++c) {
+        if (comps[c] == nullptr) {
+            throw ApiError{MHDB_INVALID_ARGUMENT, "state component must not be NULL"};
+        }
+    }
+}
+
 void ensure_staging(mhdb_solver* h)
 {
     if (h->staging == nullptr) {
@@ -1075,14 +1085,9 @@ int mhdb_upload(mhdb_solver* h, const double* const comps[9], size_t n_tot)
         if (comps == nullptr || n_tot != h->ntot) {
             throw ApiError{MHDB_INVALID_ARGUMENT, "StateField size does not match Grid2D"};
         }
+        require_components(comps);
         ensure_staging(h);
-        for (int c = 0; c < 9; ++c) {
-            if (comps[c] == nullptr) {
-                throw ApiError{MHDB_INVALID_ARGUMENT, "state component must not be NULL"};
-            }
-            MHDB_CHECK(cudaMemcpyAsync(h->staging + c * h->ntot, comps[c], h->ntot * sizeof(double),
-                                       cudaMemcpyHostToDevice, h->stream));
-        }
+        MHDB_CHECK(copy_planes(h->staging, comps, h->ntot, cudaMemcpyHostToDevice, h->stream));
         const long long n = static_cast<long long>(h->grid.nx) * h->grid.ny;
         if (h->precision == MHDB_FP64) {
             unpack_f64<<<launch_blocks(n, 256), 256, 0, h->stream>>>(
@@ -1104,6 +1109,7 @@ int mhdb_download(mhdb_solver* h, double* const comps[9], size_t n_tot)
         if (comps == nullptr || n_tot != h->ntot) {
             throw ApiError{MHDB_INVALID_ARGUMENT, "StateField size does not match Grid2D"};
         }
+        require_components(comps);
         ensure_staging(h);
         // gamma only matters for the wall fill; it is the one of the last solve.
         const double gm1 = h->last_gm1;
@@ -1124,13 +1130,7 @@ int mhdb_download(mhdb_solver* h, double* const comps[9], size_t n_tot)
             ++h->launches;
         }
         MHDB_CHECK(cudaGetLastError());
-        for (int c = 0; c < 9; ++c) {
-            if (comps[c] == nullptr) {
-                throw ApiError{MHDB_INVALID_ARGUMENT, "state component must not be NULL"};
-            }
-            MHDB_CHECK(cudaMemcpyAsync(comps[c], h->staging + c * h->ntot, h->ntot * sizeof(double),
-                                       cudaMemcpyDeviceToHost, h->stream));
-        }
+        MHDB_CHECK(copy_planes(h->staging, comps, h->ntot, cudaMemcpyDeviceToHost, h->stream));
         MHDB_CHECK(cudaStreamSynchronize(h->stream));
     });
 }
