@@ -138,8 +138,12 @@ __device__ __forceinline__ T minmod(T a, T b)
 // include/mhd/mhd_types.hpp:44). FP32 van Leer: ab * rcp(a + b) without a branch; when ab > 0
 // after rounding, a and b share their sign and max(|a|, |b|) >= 2^-74.5, so a + b is a normal
 // number and the approximate reciprocal is within its stated error; otherwise the select returns
-// 0. FP64 MC: where ab > 0 the central slope has the sign of both, so its product test is left
-// out. FP64 van Leer is limit_half_slopes below.
+// 0. FP64 van Leer the same with fast_rcp and the sign of ab read from its upper word (flat: zero,
+// negative or below 2^-1042; NaN passes; a + b is at least 2^-521 elsewhere): one reciprocal per
+// component costs three FP64 instructions and no branch, where inverting a cell's nine sums with one
+// division cost 3.5 each, a range test and a fallback (per
+// step: 1024^2 167 -> 162 us, masked non-ideal 2048^2 1.09 -> 1.03 ms). FP64 MC: where ab > 0 the
+// central slope has the sign of both, so its product test is left out.
 template <int L, class T>
 __device__ __forceinline__ T limit_half_slope(T a, T b)
 {
@@ -151,87 +155,26 @@ __device__ __forceinline__ T limit_half_slope(T a, T b)
         return (a * b <= T(0)) ? T(0) : (fabs(c) < fabs(m) ? c : m);
     } else if constexpr (L == kMC) {
         return minmod(T(0.25) * (a + b), minmod(a, b));
+    } else if constexpr (sizeof(T) == 8) {
+        const T p = a * b;
+        const int hi = __double2hiint(p);
+        const bool flat = hi <= 0 && static_cast<unsigned>(hi) <= 0xfff00000u;
+        const T q = p * fast_rcp(a + b);
+        return flat ? T(0) : q;
     } else {
-        static_assert(sizeof(T) == 4, "FP64 van Leer limits nine slopes at once");
         const float p = a * b;
         const float q = p * fast_rcp(a + b);
         return (p <= 0.0f) ? 0.0f : q;
     }
 }
 
-// 1/x for a normal or infinite FP64 x without a division: the hardware approximation
-// rcp.approx.ftz.f64 refined by two Newton-Raphson steps e = 1 - x y, y += y e (the classical
-// iteration, each step squaring the relative error), so within a few ulp of 1/x; 0 for |x| of
-// 2^1022 and above. Used only where a product of slopes left the normal range.
-__device__ __forceinline__ double newton_rcp(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    double e = fma(-x, y, 1.0);
-    y = fma(y, e, y);
-    e = fma(-x, y, 1.0);
-    return fma(y, e, y);
-}
-
-// limit_half_slope of nine components (a[c], b[c]). FP64 van Leer takes one reciprocal for all
-// nine (simultaneous inversion over a two-level product tree: groups g_j = s_3j s_3j+1 s_3j+2,
-// q = 1 / (g_0 g_1 g_2), 1/g_2 = (g_0 g_1) q, 1/g_0 = g_1 (g_2 q), 1/g_1 = g_0 (g_2 q), then the
-// same within each group; s = a + b if ab > 0 and 1 where the slope is 0 anyway), each within a
-// few ulp of 1/s. The sign of ab is read from its upper word (flat: zero, negative or below
-// 2^-1042; NaN passes). If the product leaves the range of fast_rcp, every component takes its
-// own reciprocal (newton_rcp). Every other limiter and precision: component by component.
+// limit_half_slope of nine components (a[c], b[c]).
 template <int L, class T>
 __device__ __forceinline__ void limit_half_slopes(const T (&a)[9], const T (&b)[9], T (&out)[9])
 {
-    if constexpr (L == kVanLeer && sizeof(T) == 8) {
-        T p[9], s[9], r[9];
-        bool flat[9];
 #pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            p[c] = a[c] * b[c];
-            const int hi = __double2hiint(p[c]);
-            flat[c] = hi <= 0 && static_cast<unsigned>(hi) <= 0xfff00000u;
-            s[c] = flat[c] ? T(1) : a[c] + b[c];
-        }
-        T p01[3], g[3];
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            p01[j] = s[3 * j] * s[3 * j + 1];
-            g[j] = p01[j] * s[3 * j + 2];
-        }
-        const T g01 = g[0] * g[1];
-        const T prod = g01 * g[2];
-        // 2^-1022 <= |prod| < 2^1022
-        const unsigned mag = static_cast<unsigned>(__double2hiint(prod)) & 0x7fffffffu;
-        if (mag - 0x00100000u < 0x7fc00000u) {
-            const T inv = fast_rcp(prod);
-            T ig[3];
-            ig[2] = g01 * inv;
-            const T i01 = g[2] * inv;
-            ig[0] = g[1] * i01;
-            ig[1] = g[0] * i01;
-#pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                r[3 * j + 2] = p01[j] * ig[j];
-                const T t = s[3 * j + 2] * ig[j];
-                r[3 * j] = s[3 * j + 1] * t;
-                r[3 * j + 1] = s[3 * j] * t;
-            }
-        } else {
-#pragma unroll
-            for (int c = 0; c < 9; ++c) {
-                r[c] = newton_rcp(s[c]);
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            out[c] = flat[c] ? T(0) : p[c] * r[c];
-        }
-    } else {
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            out[c] = limit_half_slope<L>(a[c], b[c]);
-        }
+    for (int c = 0; c < 9; ++c) {
+        out[c] = limit_half_slope<L>(a[c], b[c]);
     }
 }
 
@@ -279,12 +222,17 @@ __device__ __forceinline__ void conserved_and_flux(const PrimN<T>& W, T inv_gm1,
     const T mn = W.rho * W.vn;
     const T mt = W.rho * W.vt;
     const T mz = W.rho * W.vz;
-    const T v2 = W.vn * W.vn + W.vt * W.vt + W.vz * W.vz;
     const T b2 = W.bn * W.bn + W.bt * W.bt + W.bz * W.bz;
     const T pmag = T(0.5) * b2;
-    const T energy = W.p * inv_gm1 + T(0.5) * W.rho * v2 + pmag;
     const T pstar = W.p + pmag;
     const T vb = W.vn * W.bn + W.vt * W.bt + W.vz * W.bz;
+    T energy;
+    if constexpr (sizeof(T) == 8) { // rho v^2 from the momenta: two FP64 instructions fewer
+        energy = W.p * inv_gm1 + T(0.5) * (b2 + (mn * W.vn + mt * W.vt + mz * W.vz));
+    } else {
+        const T v2 = W.vn * W.vn + W.vt * W.vt + W.vz * W.vz;
+        energy = W.p * inv_gm1 + T(0.5) * W.rho * v2 + pmag;
+    }
 
     U.rho = W.rho;
     U.mn = mn;
