@@ -200,11 +200,11 @@ int mhdb_tile_config_kind(int precision, int config);
 /* mhdb_set_tile_config(h, -1) restores the default, by the grid's cells: unmasked FP32-mixed solves
    run the TMA strip march of the increment form (configuration 17) from 768 x 768 cells up and the
    one-warp register march (configuration 18) below; masked ones the TMA strip march that also
-   serves masks (configuration 11) from 1024 x 1024 up and configuration 0 below. Unmasked FP64
-   solves run the FP64 TMA strip march (configuration 7), between about 190 x 190 and 264 x 264
-   cells the 320-thread tile kernel (configuration 2; non-ideal ones configuration 0); masked ones
-   configuration 7 from 2048 x 2048 up and configuration 0 below. The strip marches cut a grid into
-   segments of at most their tile height, by the size of the grid. */
+   serves masks (configuration 11) from 600 x 600 up and configuration 0 below. Unmasked FP64
+   solves run the FP64 TMA strip march (configuration 7) from 448 x 448 cells up and the one-warp
+   register march (configuration 8) below; masked ones configuration 7 from 1200 x 1200 up and
+   configuration 0 below. The strip marches cut a grid into segments of at most their tile height,
+   by the size of the grid. */
 int mhdb_set_tile_config(mhdb_solver* h, int config);
 
 /* Additive, for tests of the error path: every bulk-copy wait of the TMA strip marches is bounded

@@ -23,22 +23,19 @@ constexpr int kCount = sizeof(kInfo) / sizeof(kInfo[0]);
 
 int stage_config_count_f64() { return kCount; }
 
-// Without a chosen configuration: unmasked FP64 grids run the TMA strip march (configuration 7),
-// whose segments are cut to the grid (segment_rows), except where the tile kernel's blocks make
-// one wave of two per SM and the march's just miss one, about 190^2 to 264^2 cells (per step at
-// 256^2: tile 22.7, march 25.5 us; at 128^2 16.5 and 15.1, at 300^2 33 and 27, at 512^2 67 and 52,
-// at 1024^2 258 and 163). There ideal solves take the 320-thread tile kernel (configuration 2),
-// non-ideal ones configuration 0. Masked grids march from 2048^2 cells up and run configuration 0
-// below (512^2 92 against 113 us, 1024^2 343 and 345, 2048^2 1294 and 1059).
-int default_stage_config_f64(long long cells, bool mask, bool nonideal)
+// Without a chosen configuration: unmasked FP64 grids run a strip march, whose segments are cut to
+// the grid (segment_rows): below 448^2 cells, where the state stays in L2 and a stage is a chain of
+// latencies, the one-warp register march (configuration 8), above the TMA march (configuration 7).
+// Per step, tile kernel (configuration 2) / register / TMA march: 128^2 15.8 / 14.0 / 15.1 us, 256^2
+// 23.3 / 24.1 / 25.7, 300x173 23.7 / 20.9 / 21.4, 400^2 48.9 / 37.9 / 38.6, 512^2 67 / 52.4 / 51.1,
+// 1024^2 258 / 204 / 162. Masked grids march from 1200^2 cells up and run the tile kernel
+// (configuration 0) below: 512^2 83 against 105 us, 1024^2 304 and 313, 1448^2 594 and 506.
+int default_stage_config_f64(long long cells, bool mask)
 {
     if (mask) {
-        return cells >= 2048LL * 2048 ? 7 : 0;
+        return cells >= 1200LL * 1200 ? 7 : 0;
     }
-    if (cells >= 190LL * 190 && cells < 264LL * 264) {
-        return nonideal ? 0 : 2;
-    }
-    return 7;
+    return cells >= 448LL * 448 ? 7 : 8;
 }
 
 TileConfigInfo stage_config_info_f64(int c) { return kInfo[c < 0 || c >= kCount ? 0 : c]; }

@@ -44,14 +44,15 @@ int stage_config_count_mixed() { return kCount; }
 // the increment form with stage 2's own-cell increment taken from the halo stream (configuration
 // 17); smaller ones, whose state stays in L2, the one-warp register march of the stored form
 // (configuration 18), which has no copies to set up (per step, register against TMA march: 128^2
-// 13.4 and 14.3, 360^2 22.2 and 25.2, 512^2 38 and 39, 640^2 49 and 50, 724^2 56 and 56, 900^2 90
-// and 84, 1024^2 110 and 99 us; the tile kernel took 18.5, 24.9, 46 and 168 us at 128^2, 360^2,
-// 512^2 and 1024^2). Masked grids of at least 1024^2 cells run the stored-form TMA march
-// (configuration 11), smaller ones the tile kernel.
+// 13.7 and 15.2 us, 301x173 17.1 and 19.2, 400^2 26.6 and 29.6, 512^2 38 and 40, 640^2 49 and 50,
+// 724^2 56 and 56, 900^2 90 and 84, 1024^2 110 and 99; the tile kernel took 18.5, 21.5, 36, 46 and
+// 168 us at 128^2, 301x173, 400^2, 512^2 and 1024^2). Masked grids of at least 600^2 cells run the
+// stored-form TMA march (configuration 11), smaller ones the tile kernel (512^2 74 against 68 us,
+// 724^2 102 against 117).
 int default_stage_config_mixed(long long cells, bool mask)
 {
     if (mask) {
-        return cells >= 1024LL * 1024 ? 11 : 0;
+        return cells >= 600LL * 600 ? 11 : 0;
     }
     return cells >= 768LL * 768 ? 17 : 18;
 }

@@ -420,7 +420,7 @@ StepPlan make_plan(mhdb_solver* h, const mhdb_params* p)
     // solve the chosen configuration does not serve (e.g. a masked solve after an autotuner
     // choice made on unmasked grids) uses the default configuration of its size, else 0.
     const long long cells = static_cast<long long>(h->grid.nx) * h->grid.ny;
-    const int dflt = h->precision == MHDB_FP64 ? default_stage_config_f64(cells, h->has_mask, ni)
+    const int dflt = h->precision == MHDB_FP64 ? default_stage_config_f64(cells, h->has_mask)
                                                : default_stage_config_mixed(cells, h->has_mask);
     auto serves = [&](int c) {
         return c == 0 || (h->precision == MHDB_FP64

@@ -57,7 +57,7 @@ int stage_config_count_mixed();
 // most `most` rows, of which `slots` are resident on the GPU (solver.cu).
 int segment_rows(int nx, int ny, int tile_x, int most, int slots);
 // Configuration used when none is chosen (mhdb_set_tile_config(h, -1), the default).
-int default_stage_config_f64(long long cells, bool mask, bool nonideal);
+int default_stage_config_f64(long long cells, bool mask);
 int default_stage_config_mixed(long long cells, bool mask);
 TileConfigInfo stage_config_info_f64(int config);
 TileConfigInfo stage_config_info_mixed(int config);
