@@ -125,31 +125,35 @@ struct LoadMxParity {
     }
 };
 
-template <int NT, class Load, class Speed>
-__global__ void batch_cfl_init(Load load, Speed speed, Geometry g, Consts k, Ctrl* ctrl)
+template <int NT, class Speed>
+__global__ void batch_cfl_init(Speed speed, Geometry g, Consts k, Ctrl* ctrl)
 {
     double smax = 0.0;
     const long long ncell = static_cast<long long>(g.nx) * g.ny;
     for (long long c = blockIdx.x * static_cast<long long>(NT) + threadIdx.x; c < ncell;
          c += static_cast<long long>(gridDim.x) * NT) {
         const int x = static_cast<int>(c % g.nx), y = static_cast<int>(c / g.nx);
-        double r[9];
-        load(x, y, r);
-        smax = vmax(smax, speed(r, k));
+        smax = vmax(smax, speed(x, y, k));
     }
     reduce_signal_speed_and_finish(smax, ctrl, k, gridDim.x, false);
 }
 
 struct SpeedF64 {
-    __device__ double operator()(const double* r, const Consts& k) const
+    const double* u;
+    Geometry g;
+    __device__ double operator()(int x, int y, const Consts& k) const
     {
+        double r[9];
+        load_cons_f64(u, g, x, y, r);
         return PolicyF64::signal_speed(r, k);
     }
 };
 struct SpeedMx {
-    __device__ double operator()(const double* r, const Consts& k) const
+    MixedState u;
+    Geometry g;
+    __device__ double operator()(int x, int y, const Consts& k) const
     {
-        return PolicyMixed::signal_speed(r, k);
+        return PolicyMixed::signal_speed_hi(u, g, x, y, k);
     }
 };
 
@@ -863,10 +867,10 @@ void add_solve(mhdb_batch* b, const mhdb_grid* grid, const mhdb_params* params, 
     const int init_blocks = static_cast<int>(std::min<long long>((n + kInitThreads - 1) / kInitThreads, 148LL * 4));
     if (b->precision == MHDB_FP64) {
         batch_cfl_init<kInitThreads><<<init_blocks, kInitThreads, 0, b->stream>>>(
-            LoadF64{static_cast<const double*>(s.U), s.geom}, SpeedF64{}, s.geom, s.k, b->ctrl + slot);
+            SpeedF64{static_cast<const double*>(s.U), s.geom}, s.geom, s.k, b->ctrl + slot);
     } else {
         batch_cfl_init<kInitThreads><<<init_blocks, kInitThreads, 0, b->stream>>>(
-            LoadMx{mixed_view(s.U, s.geom), s.geom}, SpeedMx{}, s.geom, s.k, b->ctrl + slot);
+            SpeedMx{mixed_view(s.U, s.geom), s.geom}, s.geom, s.k, b->ctrl + slot);
     }
     ++b->launches;
     check(cudaGetLastError(), "batch cfl launch");
