@@ -512,12 +512,12 @@ void rebuild(mhdb_batch* b)
         }
         const size_t grid = static_cast<size_t>(sms) * b->resident_ctas[variant][ni ? 1 : 0][1];
         b->lists.push_back({variant, limiter, ni, static_cast<int>(work.size()), kv.second.count});
-        // The CTAs walk a list with a grid stride. Highest items first, and every second round of the
-        // grid in reverse (counted from the last, which may be partial), so that a CTA with a high item
-        // in one round has a low one, or none, in the next. (In
-        // list order 15 of 2383 items opened a second full round for a batch of 16 uneven solves: 292 us
-        // per step against 251; counted for batches of 16 to 256 solves, the busiest CTA is within 2 % of
-        // the best assignment's.)
+        // The CTAs walk a list with a grid stride. Highest items first, and every second round of
+        // the grid in reverse (counted from the last, which may be partial), so that a CTA with a
+        // high item in one round has a low one, or none, in the next. In list order 15 of 2383
+        // items opened a second full round for a batch of 16 uneven solves: 292 us per step against
+        // 251. Counted for batches of 16 to 256 solves, the busiest CTA is within 2 % of the best
+        // assignment's.
         const size_t first = work.size();
         for (int h = kMaxItemRows; h >= 0; --h) {
             work.insert(work.end(), kv.second.by_height[h].begin(), kv.second.by_height[h].end());

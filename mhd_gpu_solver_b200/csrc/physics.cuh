@@ -46,9 +46,9 @@ __device__ __forceinline__ bool positive_finite(double x)
 // 0.38 x 2^-53, as the IEEE division), the roots within 1.5 x 2^-53 (mean 0.38). The FP64 kernels
 // are bound by the FP64 pipe and its latencies; unlike the compiler's division and square root
 // these have no branch to a slow path, so the scheduler can interleave the chains of a face, and
-// about half the FP64 instructions. With the fast speed's one reciprocal root (below) and integer
-// sign tests, a 4096^2 van Leer step went from 2.78 to 2.21 ms, a masked non-ideal 2048^2 step
-// from 1.33 to 1.06 ms. Valid for normal operands (densities, sR - sL, fast-speed
+// about half the FP64 instructions. With the fast speed's one reciprocal root, the limiter's
+// reciprocal per component (below) and integer sign tests, a 4096^2 van Leer step went from 2.72
+// to 2.16 ms, a masked non-ideal 2048^2 step from 1.33 to 1.03 ms. Valid for normal operands (densities, sR - sL, fast-speed
 // discriminants); outside them the result is not finite, as the states that lead there are not.
 // FP32 (the FP32-mixed form): the hardware approximations rcp.approx.ftz / sqrt.approx.ftz (PTX
 // ISA; about 1 ulp), used only where the operand is a positive normal number or the result is
@@ -139,11 +139,11 @@ __device__ __forceinline__ T minmod(T a, T b)
 // after rounding, a and b share their sign and max(|a|, |b|) >= 2^-74.5, so a + b is a normal
 // number and the approximate reciprocal is within its stated error; otherwise the select returns
 // 0. FP64 van Leer the same with fast_rcp and the sign of ab read from its upper word (flat: zero,
-// negative or below 2^-1042; NaN passes; a + b is at least 2^-521 elsewhere): one reciprocal per
-// component costs three FP64 instructions and no branch, where inverting a cell's nine sums with one
-// division cost 3.5 each, a range test and a fallback (per
-// step: 1024^2 167 -> 162 us, masked non-ideal 2048^2 1.09 -> 1.03 ms). FP64 MC: where ab > 0 the
-// central slope has the sign of both, so its product test is left out.
+// negative or below 2^-1042; NaN passes; a + b is at least 2^-521 elsewhere): a reciprocal per
+// component costs three FP64 instructions and no branch, where inverting a cell's nine sums with
+// one division cost 3.5 each, a range test and a fallback (per step: 1024^2 167 -> 162 us, masked
+// non-ideal 2048^2 1.09 -> 1.03 ms). FP64 MC: where ab > 0 the central slope has the sign of both,
+// so its product test is left out.
 template <int L, class T>
 __device__ __forceinline__ T limit_half_slope(T a, T b)
 {

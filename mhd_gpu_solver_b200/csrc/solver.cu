@@ -383,7 +383,7 @@ namespace mhdb {
 // about 1.3 rows each. With w = blocks / slots, a row takes 1 + w of a lone block's time up to one
 // full wave (measured from w = 0.1 to 1 in both precision forms); beyond, 2 w and the idle part of
 // the last wave, which costs less the more waves there are. Measured per step, 32-row segments ->
-// this rule: FP32-mixed 512^2 100 -> 39 us, 1024^2 127 -> 100 us; FP64 512^2 134 -> 53 us,
+// this rule: FP32-mixed 512^2 100 -> 39 us, 1024^2 127 -> 100 us; FP64 512^2 134 -> 51 us,
 // 1448^2 342 -> 300 us; from 2048^2 up within 3 % of 32 rows.
 int segment_rows(int nx, int ny, int tile_x, int most, int slots)
 {
