@@ -32,10 +32,10 @@ __device__ __forceinline__ bool vanishes(double x)
     const int hi = __double2hiint(x);
     return hi < 0x00100000 && static_cast<unsigned>(hi) <= 0xfff00000u;
 }
-// Whether x is positive and finite (above the smallest subnormals), by its upper word.
-__device__ __forceinline__ bool positive_finite(double x)
+// Whether x lies in [2^-440, 2^440), by its upper word.
+__device__ __forceinline__ bool moderate(double x)
 {
-    return static_cast<unsigned>(__double2hiint(x)) - 1u < 0x7fefffffu;
+    return static_cast<unsigned>(__double2hiint(x)) - 0x24700000u < 0x37000000u;
 }
 
 // Reciprocal and square root.
@@ -48,8 +48,9 @@ __device__ __forceinline__ bool positive_finite(double x)
 // these have no branch to a slow path, so the scheduler can interleave the chains of a face, and
 // about half the FP64 instructions. With the fast speed's one reciprocal root, the limiter's
 // reciprocal per component (below) and integer sign tests, a 4096^2 van Leer step went from 2.72
-// to 2.16 ms, a masked non-ideal 2048^2 step from 1.33 to 1.03 ms. Valid for normal operands (densities, sR - sL, fast-speed
-// discriminants); outside them the result is not finite, as the states that lead there are not.
+// to 2.16 ms, a masked non-ideal 2048^2 step from 1.33 to 1.03 ms. For operands whose reciprocal is normal too: others
+// take rcp_any and sqrt_any, lose the result in a select, or give the NaN that the cell comes to in
+// any case (a density that is zero, subnormal or infinite).
 // FP32 (the FP32-mixed form): the hardware approximations rcp.approx.ftz / sqrt.approx.ftz (PTX
 // ISA; about 1 ulp), used only where the operand is a positive normal number or the result is
 // discarded by a select (inverse densities, 1/(sR - sL) with sR - sL >= 2 c_h, |B|, the van
@@ -66,6 +67,22 @@ __device__ __forceinline__ float fast_rcp(float x)
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+}
+// 1/x of any x: an operand that is zero, infinite or NaN gives what the division gives (the
+// approximation has these right, its correction has not), a subnormal one infinity, and one above
+// 2^1022 zero.
+__device__ __forceinline__ double rcp_any(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    const double r = fma(y, fma(e, e, e), y);
+    const bool normal = (static_cast<unsigned>(__double2hiint(x)) << 1) - 0x00200000u < 0xff800000u;
+    return normal ? r : y;
+}
+__device__ __forceinline__ float rcp_any(float x)
+{
+    return fast_rcp(x);
 }
 // a / sqrt(x), corrected as a y (1 + e/2 + 3 e^2/8), so that a factor costs nothing extra.
 __device__ __forceinline__ double scaled_rsqrt(double a, double x)
@@ -86,11 +103,21 @@ __device__ __forceinline__ double sqrt_or_zero(double x)
     const double r = fma(t * e, fma(0.375, e, 0.5), t);
     return vanishes(x) ? 0.0 : r;
 }
+// sqrt(x) of any x >= 0 or NaN: infinity and NaN as they are; a subnormal one counts as zero.
+__device__ __forceinline__ double sqrt_any(double x)
+{
+    const double r = sqrt_or_zero(x);
+    return __double2hiint(x) >= 0x7ff00000 ? x : r;
+}
 __device__ __forceinline__ float fast_sqrt(float x)
 {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
+}
+__device__ __forceinline__ float sqrt_any(float x)
+{
+    return fast_sqrt(x);
 }
 
 // mhd::simd scalar min/max (include/mhd/simd.hpp:40-47): the first operand wins ties and
@@ -178,40 +205,48 @@ __device__ __forceinline__ void limit_half_slopes(const T (&a)[9], const T (&b)[
     }
 }
 
-// Fast magnetosonic speed along n; include/mhd/kernels/muscl_hll.hpp:70-87. FP32 follows the
-// reference's form from 1/rho. FP64 factors the density out: with A = gamma p + B^2,
-// c_f = sqrt((A + sqrt(A^2 - 4 gamma p B_n^2)) / (2 rho)) = X / sqrt(2 rho X) with
-// X = A + sqrt(...), which needs one reciprocal root in place of a division and a root (and takes
-// the sign of rho into the inner root, as dividing by it does); 0 where the argument vanishes or
-// is negative.
+// Fast magnetosonic speed along n in the reference's form, from 1/rho;
+// include/mhd/kernels/muscl_hll.hpp:70-87.
 template <class T>
-__device__ __forceinline__ T fast_speed_n_inv(const PrimN<T>& W, T inv_rho, T gamma)
+__device__ __forceinline__ T reference_fast_speed(const PrimN<T>& W, T inv_rho, T gamma)
 {
-    if constexpr (sizeof(T) == 8) {
-        const T gp = gamma * W.p;
-        const T bn2 = W.bn * W.bn;
-        const T A = gp + (bn2 + W.bt * W.bt + W.bz * W.bz);
-        const T root = sqrt_or_zero(A * A - (T(4) * gp) * bn2);
-        const T X = A + copysign(root, W.rho);
-        const T arg = (W.rho + W.rho) * X;
-        const T cf = scaled_rsqrt(fabs(X), arg);
-        return vanishes(arg) ? T(0) : cf;
-    } else {
-        const T cs2 = gamma * W.p * inv_rho;
-        const T bn2 = W.bn * W.bn;
-        const T b2 = bn2 + W.bt * W.bt + W.bz * W.bz;
-        const T va2 = b2 * inv_rho;
-        const T van2 = bn2 * inv_rho;
-        const T sum = cs2 + va2;
-        const T disc = vmax(sum * sum - T(4) * cs2 * van2, T(0));
-        const T cf2 = T(0.5) * (sum + fast_sqrt(disc));
-        return fast_sqrt(vmax(cf2, T(0)));
-    }
+    const T cs2 = gamma * W.p * inv_rho;
+    const T bn2 = W.bn * W.bn;
+    const T b2 = bn2 + W.bt * W.bt + W.bz * W.bz;
+    const T va2 = b2 * inv_rho;
+    const T van2 = bn2 * inv_rho;
+    const T sum = cs2 + va2;
+    const T disc = vmax(sum * sum - T(4) * cs2 * van2, T(0));
+    const T cf2 = T(0.5) * (sum + sqrt_any(disc));
+    return sqrt_any(vmax(cf2, T(0)));
 }
-template <class T>
-__device__ __forceinline__ T fast_speed_n(const PrimN<T>& W, T gamma)
+
+// The same of an FP64 state whose density and pressure are moderate. The density is factored out:
+// with A = gamma p + B^2, c_f = sqrt((A + sqrt(A^2 - 4 gamma p B_n^2)) / (2 rho)) =
+// X / sqrt(2 rho X) with X = A + sqrt(...), which needs one reciprocal root in place of a division
+// and a root. A^2 and rho X stay normal then: gamma p >= 2^-440, and a B^2 above 2^512 leaves a
+// pressure computed from the energy beside it no value between 0 and 2^440 (its steps are 2^-53 of
+// the energy). Other states (vanishing and negative densities and pressures, infinities, NaN,
+// extreme units) take the reference's form, so that a speed that overflows is infinite here too.
+__device__ __forceinline__ double moderate_fast_speed(const PrimN<double>& W, double gamma)
 {
-    return fast_speed_n_inv(W, fast_rcp(W.rho), gamma);
+    const double gp = gamma * W.p;
+    const double bn2 = W.bn * W.bn;
+    const double A = gp + (bn2 + W.bt * W.bt + W.bz * W.bz);
+    const double X = A + sqrt_or_zero(A * A - (4.0 * gp) * bn2);
+    return scaled_rsqrt(X, (W.rho + W.rho) * X);
+}
+
+// Fast speeds of a face's FP64 states that are not moderate. They are found in the branch that
+// chooses the states and taken by a select: a branch around the speeds, or a general flux beside the
+// usual one, splits the face's arithmetic and costs 4 to 10 % of a step, this costs 0 to 3 %.
+struct GivenSpeeds {
+    bool given = false;
+    double left = 0.0, right = 0.0;
+};
+__device__ __forceinline__ bool moderate_states(const PrimN<double>& L, const PrimN<double>& R)
+{
+    return moderate(L.rho) && moderate(L.p) && moderate(R.rho) && moderate(R.p);
 }
 
 // Conserved state and GLM-MHD flux along n; include/mhd/kernels/muscl_hll.hpp:89-124.
@@ -261,12 +296,20 @@ __device__ __forceinline__ void conserved_and_flux(const PrimN<T>& W, T inv_gm1,
 
 // HLL flux with Dedner GLM wave-speed bounds (-c_h, +c_h) from the two face states, with the
 // upwind and degenerate (|sR - sL| < 1e-14) branches; include/mhd/kernels/muscl_hll.hpp:170-208.
+// speeds: the fast speeds of FP64 states that are not moderate.
 template <class T>
 __device__ __forceinline__ FluxN<T> hll_flux(const PrimN<T>& WL, const PrimN<T>& WR, T gamma,
-                                             T inv_gm1, T c_h)
+                                             T inv_gm1, T c_h, const GivenSpeeds& speeds)
 {
-    const T cfL = fast_speed_n(WL, gamma);
-    const T cfR = fast_speed_n(WR, gamma);
+    T cfL, cfR;
+    if constexpr (sizeof(T) == 8) {
+        const T fL = moderate_fast_speed(WL, gamma), fR = moderate_fast_speed(WR, gamma);
+        cfL = speeds.given ? speeds.left : fL;
+        cfR = speeds.given ? speeds.right : fR;
+    } else {
+        cfL = reference_fast_speed(WL, fast_rcp(WL.rho), gamma);
+        cfR = reference_fast_speed(WR, fast_rcp(WR.rho), gamma);
+    }
     const T sL = vmin(vmin(WL.vn - cfL, WR.vn - cfR), -c_h);
     const T sR = vmax(vmax(WL.vn + cfL, WR.vn + cfR), c_h);
 
@@ -324,7 +367,7 @@ template <class T>
 __device__ __forceinline__ T cell_max_signal_speed(T rho, T mx, T my, T mz, T energy, T bx, T by,
                                                    T bz, T gamma)
 {
-    const T inv_rho = fast_rcp(rho);
+    const T inv_rho = rcp_any(rho);
     PrimN<T> W;
     W.rho = rho;
     W.vn = mx * inv_rho;
@@ -337,13 +380,25 @@ __device__ __forceinline__ T cell_max_signal_speed(T rho, T mx, T my, T mz, T en
     W.bt = by;
     W.bz = bz;
     W.psi = T(0);
-    const T sx = fabs(W.vn) + fast_speed_n_inv(W, inv_rho, gamma);
     PrimN<T> Wy = W;
     Wy.vn = W.vt;
     Wy.vt = W.vn;
     Wy.bn = by;
     Wy.bt = bx;
-    const T sy = fabs(Wy.vn) + fast_speed_n_inv(Wy, inv_rho, gamma);
+    T cx, cy;
+    if constexpr (sizeof(T) == 8) {
+        cx = moderate_fast_speed(W, gamma);
+        cy = moderate_fast_speed(Wy, gamma);
+        if (__builtin_expect(!(moderate(rho) && moderate(W.p)), 0)) {
+            cx = reference_fast_speed(W, inv_rho, gamma);
+            cy = reference_fast_speed(Wy, inv_rho, gamma);
+        }
+    } else {
+        cx = reference_fast_speed(W, inv_rho, gamma);
+        cy = reference_fast_speed(Wy, inv_rho, gamma);
+    }
+    const T sx = fabs(W.vn) + cx;
+    const T sy = fabs(Wy.vn) + cy;
     return vmax(sx, sy);
 }
 

@@ -109,20 +109,33 @@ __device__ __forceinline__ void face_flux_regs(const T (&lc)[9], const T (&sl)[9
     // physical component feeding each rotated-frame slot (rho, vn, vt, vz, p, bn, bt, bz, psi)
     constexpr int comp[9] = {0, YDIR ? 2 : 1, YDIR ? 1 : 2, 3, 4, YDIR ? 6 : 5, YDIR ? 5 : 6, 7, 8};
     T l[9], r[9];
+    GivenSpeeds speeds;
     if constexpr (sizeof(T) == 8) {
-        // The second-order states, and the first-order ones only where a density or pressure
-        // fails the test.
+        // The second-order states; where a density or pressure is not moderate, the test, the
+        // first-order states, and the speeds of states that are not moderate either.
 #pragma unroll
         for (int q = 0; q < 9; ++q) {
             l[q] = lc[comp[q]] + sl[comp[q]];
             r[q] = rc[comp[q]] - sr[comp[q]];
         }
-        if (!(positive_finite(l[0]) && positive_finite(l[4]) && positive_finite(r[0]) &&
-              positive_finite(r[4]))) {
+        const PrimN<T> L2{l[0], l[1], l[2], l[3], l[4], l[5], l[6], l[7], l[8]};
+        const PrimN<T> R2{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8]};
+        if (__builtin_expect(!moderate_states(L2, R2), 0)) {
+            const T inf = T(INFINITY);
+            if (!((l[0] > T(0)) && (l[4] > T(0)) && (l[0] < inf) && (l[4] < inf) && (r[0] > T(0)) &&
+                  (r[4] > T(0)) && (r[0] < inf) && (r[4] < inf))) {
 #pragma unroll
-            for (int q = 0; q < 9; ++q) {
-                l[q] = lc[comp[q]];
-                r[q] = rc[comp[q]];
+                for (int q = 0; q < 9; ++q) {
+                    l[q] = lc[comp[q]];
+                    r[q] = rc[comp[q]];
+                }
+            }
+            const PrimN<T> L{l[0], l[1], l[2], l[3], l[4], l[5], l[6], l[7], l[8]};
+            const PrimN<T> R{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8]};
+            if (__builtin_expect(!moderate_states(L, R), 0)) {
+                speeds.given = true;
+                speeds.left = reference_fast_speed(L, rcp_any(L.rho), gamma);
+                speeds.right = reference_fast_speed(R, rcp_any(R.rho), gamma);
             }
         }
     } else {
@@ -143,7 +156,7 @@ __device__ __forceinline__ void face_flux_regs(const T (&lc)[9], const T (&sl)[9
     }
     const PrimN<T> WL{l[0], l[1], l[2], l[3], l[4], l[5], l[6], l[7], l[8]};
     const PrimN<T> WR{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8]};
-    const FluxN<T> f = hll_flux(WL, WR, gamma, inv_gm1, c_h);
+    const FluxN<T> f = hll_flux(WL, WR, gamma, inv_gm1, c_h, speeds);
     out[0] = f.rho;
     out[1] = YDIR ? f.mt : f.mn;
     out[2] = YDIR ? f.mn : f.mt;
