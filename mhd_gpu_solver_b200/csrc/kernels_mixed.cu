@@ -40,21 +40,23 @@ constexpr int kCount = sizeof(kInfo) / sizeof(kInfo[0]);
 
 int stage_config_count_mixed() { return kCount; }
 
-// Without a chosen configuration: unmasked grids of at least 768^2 cells run the TMA strip march of
+// Without a chosen configuration: unmasked grids of at least 1024^2 cells run the TMA strip march of
 // the increment form with stage 2's own-cell increment taken from the halo stream (configuration
-// 17); smaller ones, whose state stays in L2, the one-warp register march of the stored form
-// (configuration 18), which has no copies to set up (per step, register against TMA march: 128^2
-// 13.7 and 15.2 us, 301x173 17.1 and 19.2, 400^2 26.6 and 29.6, 512^2 38 and 40, 640^2 49 and 50,
-// 724^2 56 and 56, 900^2 90 and 84, 1024^2 110 and 99; the tile kernel took 18.5, 21.5, 36, 46 and
-// 168 us at 128^2, 301x173, 400^2, 512^2 and 1024^2). Masked grids of at least 600^2 cells run the
-// stored-form TMA march (configuration 11), smaller ones the tile kernel (512^2 74 against 68 us,
-// 724^2 102 against 117).
+// 17); smaller ones the one-warp register march of the stored form (configuration 18), which has no
+// copies to set up (per step, register against TMA march: 128^2 13.7 and 15.2 us, 301x173 17.1 and
+// 19.2, 400^2 26.6 and 29.6, 512^2 38 and 40, 640^2 49 and 50, 724^2 56 and 56; the tile kernel took
+// 18.5, 21.5, 36, 46 and 168 us at 128^2, 301x173, 400^2, 512^2 and 1024^2). From 724^2 up the TMA
+// march is the faster one (900^2 90 and 84 us, 1024^2 110 and 99), but the increment form rounds
+// U* - U^n to FP32 where the stored form keeps U* as a hi + lo pair, and its error against FP64 is 10
+// to 16 % larger (800x760: 2.9e-8 against 2.6e-8), so it serves only the sizes it was chosen for.
+// Masked grids of at least 600^2 cells run the stored-form TMA march (configuration 11), smaller
+// ones the tile kernel (512^2 74 against 68 us, 724^2 102 against 117).
 int default_stage_config_mixed(long long cells, bool mask)
 {
     if (mask) {
         return cells >= 600LL * 600 ? 11 : 0;
     }
-    return cells >= 768LL * 768 ? 17 : 18;
+    return cells >= 1024LL * 1024 ? 17 : 18;
 }
 
 TileConfigInfo stage_config_info_mixed(int c) { return kInfo[c < 0 || c >= kCount ? 0 : c]; }
