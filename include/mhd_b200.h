@@ -200,7 +200,7 @@ int mhdb_tile_config_kind(int precision, int config);
 /* mhdb_set_tile_config(h, -1) restores the default, by the grid's cells: unmasked FP32-mixed solves
    run the TMA strip march of the increment form (configuration 17) from 1024 x 1024 cells up and the
    one-warp register march (configuration 18) below; masked ones the TMA strip march that also
-   serves masks (configuration 11) from 600 x 600 up and configuration 0 below. Unmasked FP64
+   serves masks (configuration 11) from 1024 x 1024 up and configuration 0 below. Unmasked FP64
    solves run the FP64 TMA strip march (configuration 7) from 448 x 448 cells up and the one-warp
    register march (configuration 8) below; masked ones configuration 7 from 1200 x 1200 up and
    configuration 0 below. The strip marches cut a grid into segments of at most their tile height,

@@ -49,12 +49,14 @@ int stage_config_count_mixed() { return kCount; }
 // march is the faster one (900^2 90 and 84 us, 1024^2 110 and 99), but the increment form rounds
 // U* - U^n to FP32 where the stored form keeps U* as a hi + lo pair, and its error against FP64 is 10
 // to 16 % larger (800x760: 2.9e-8 against 2.6e-8), so it serves only the sizes it was chosen for.
-// Masked grids of at least 600^2 cells run the stored-form TMA march (configuration 11), smaller
-// ones the tile kernel (512^2 74 against 68 us, 724^2 102 against 117).
+// Masked grids of at least 1024^2 cells run the stored-form TMA march (configuration 11), smaller
+// ones the tile kernel: the march stores a solid cell from the row's FP32 primitives, the tile kernel
+// from the FP64 wall fill, so the march stays with the sizes it was chosen for (512^2 74 against 68
+// us, 724^2 102 against 117).
 int default_stage_config_mixed(long long cells, bool mask)
 {
     if (mask) {
-        return cells >= 600LL * 600 ? 11 : 0;
+        return cells >= 1024LL * 1024 ? 11 : 0;
     }
     return cells >= 1024LL * 1024 ? 17 : 18;
 }

@@ -30,3 +30,31 @@ def test_default_keeps_the_intermediate_state_as_a_pair(nx, ny, nonideal):
     err = [np.linalg.norm(interior(gpu_solve(U0, grid, p, precision=_capi.FP32,
                                              tile_config=c)[0]) - want) for c in (-1, 0)]
     assert err[0] <= 1.02 * err[1], (err, np.linalg.norm(want))
+
+
+@pytest.mark.parametrize("nx,ny", [(130, 150), (640, 600), (1000, 900)])
+def test_default_stores_solid_cells_from_the_fp64_fill(nx, ny):
+    """Below 1024^2 cells a solid cell is stored from the FP64 wall fill of the whole hi + lo state: the
+    fluid neighbour's values with the normal momentum negated, exactly representable as a pair. After
+    one step with dt so small that nothing else moves in FP32, a solid cell whose fluid neighbour is
+    +x holds that neighbour's tangential momentum, energy and field to the pair's 2^-48 instead of
+    FP32's 2^-24. The stored values are seen where the mask is taken off before the download, which
+    fills solid cells anew."""
+    mask = wl.circles_and_rectangles(nx, ny, 0)
+    U0 = initial_state(wl.fourier_state(nx, ny, 3), 5.0 / 3.0, mask=mask)
+    dev = _capi.DeviceSolver(nx, ny, precision=_capi.FP32)
+    try:
+        dev.configure(_capi.BC_PERIODIC, _capi.BC_PERIODIC, mask)
+        dev.upload(U0)
+        dev.solve_steps(_capi.make_params(limiter=_capi.VANLEER, cfl=1e-12), 1)
+        dev.configure(_capi.BC_PERIODIC, _capi.BC_PERIODIC, None)
+        got = interior(dev.download())
+    finally:
+        dev.close()
+    solid, fluid_right = mask[:, :-1] == 0, mask[:, 1:] != 0
+    at = solid & fluid_right
+    assert at.sum() > 20
+    for c in (0, 2, 4, 5, 6):
+        s, f = got[c][:, :-1][at], got[c][:, 1:][at]
+        scale = np.abs(got[c]).max()
+        assert np.abs(s - f).max() <= 1e-10 * scale, (c, np.abs(s - f).max() / scale)
