@@ -299,7 +299,8 @@ int mhdb_batch_poll(mhdb_batch* b, int* active);
    (tile width and height), its threads and its kernel kind (MHDB_KERNEL_*). FP32-mixed: 0 = TMA
    strip march, one warp by 32 rows; 1 = register strip march, 4 warps by 32 rows; 2 = TMA strip
    march, one warp by 64 rows; 3 = TMA strip march of the increment form, one warp by 32 rows
-   (the default). Solves of fewer than 128 x 128 cells take 16 rows in place of 32.
+   (the default for solves of at least 128 x 128 cells; smaller ones take 0, and 8 rows in place
+   of 32).
    mhdb_batch_set_config picks one for a solve (-1: by the solve's size, the default); once a
    solve has been stepped it cannot change between configuration 3 and the others
    (MHDB_INVALID_ARGUMENT). The batch autotuner (mhd_gpu_solver_b200.autotune.tune_batch) chooses

@@ -198,15 +198,16 @@ struct BatchVariant {
     int tile_x, tile_y, threads, kind; // kind: MHDB_KERNEL_*
 };
 
-// Rows of a solve's work items. A march item is a serial chain of its rows: a batch of a few small
-// solves ends with its longest chain (64 solves of 64^2, per step: 32-row items 128 us, 16-row ones
-// 83), a full one pays for finer items' prologues (64 solves of sides 64-1024: 916 us with 32 rows,
-// 1056 with 16 below 1024^2). The rule sees the solve alone, never the mix: a solve's values do not
-// depend on the other solves.
+// Rows of a solve's work items. A march item is a serial chain of its rows, and a list ends with its
+// longest chain; finer items pay for their prologues once the list fills the GPU. Small solves (a list
+// of their own by default), per step with 16 / 8 / 4 rows: one of 64^2 63 / 37 / 25 us, 64 of them
+// 75 / 55 / 67, 256 of them 196 / 211 / 246; 16 solves of sides 64-1024 415 / 389 / 376. Larger ones:
+// 64 of sides 64-1024 916 us with 32 rows, 1056 with 16 below 1024^2. The rule sees the solve alone,
+// never the mix: a solve's values do not depend on the other solves.
 int item_rows(const BatchVariant& v, const mhdb_grid& g)
 {
     const long long cells = static_cast<long long>(g.nx) * g.ny;
-    return v.tile_y == 32 && cells < 128LL * 128 ? 16 : v.tile_y;
+    return v.tile_y == 32 && cells < 128LL * 128 ? 8 : v.tile_y;
 }
 
 constexpr int kMaxItemRows = 64; // of any configuration
@@ -255,10 +256,12 @@ struct BatchKernels<PolicyMixed> {
         if (v == 3) return {kMarchOwned, 32, 32, MHDB_KERNEL_MARCH_TMA_DELTA};
         return {kMarchOwned, 32, 32, MHDB_KERNEL_MARCH_TMA};
     }
-    // The increment form for every size: lists of one configuration share a launch per stage, so a
-    // small solve's items run beside the others' (in the register march of configuration 1, and a
-    // launch of its own, one solve under 128^2 cells cost 180 us per step).
-    static int default_variant(long long) { return kDeltaVariant; }
+    // The increment form from 128^2 cells up; smaller solves keep U* as a hi + lo pair (TMA march of
+    // the stored form; the increment form's error against FP64 is about a tenth larger), in a list
+    // and launches of their own: in the increment form's list 16 solves of sides 64-1024 took 348 us
+    // per step, this way 389, 64 of them 1000 and 1035, 64 solves of 64^2 alone 82 and 55. As the
+    // default before, configuration 1 needs 407, 1054 and 53.
+    static int default_variant(long long cells) { return cells >= 128LL * 128 ? kDeltaVariant : 0; }
     template <int L, bool NI, int STAGE>
     static Fn fn(int v)
     {
