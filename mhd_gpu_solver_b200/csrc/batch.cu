@@ -355,12 +355,12 @@ struct mhdb_batch {
         int limiter;
         bool ni;
         int offset, count;
+        int ctas; // resident CTAs per SM of both stages' kernels: the work order follows this grid
     };
     std::vector<List> lists;
     bool dirty = true;
     size_t bytes_in_use = 0;
     long long launches = 0;
-    int resident_ctas[4][2][2] = {}; // [variant][ni][stage-1] CTAs per SM
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
 };
@@ -503,7 +503,7 @@ void rebuild(mhdb_batch* b)
     for (auto& kv : items) {
         const int variant = std::get<0>(kv.first), limiter = std::get<1>(kv.first);
         const bool ni = std::get<2>(kv.first) != 0;
-        // CTAs per SM of the kernels (occupancy of the persistent grid)
+        int ctas = 0;
         for (int st = 1; st <= 2; ++st) {
             auto fn = batch_fn<Policy>(variant, limiter, ni, st);
             const size_t sm = K::smem(variant, ni, st);
@@ -511,10 +511,11 @@ void rebuild(mhdb_batch* b)
                   "cudaFuncSetAttribute");
             int nb = 0;
             check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, K::variant(variant).threads, sm), "occupancy");
-            b->resident_ctas[variant][ni ? 1 : 0][st - 1] = std::max(1, nb);
+            ctas = st == 1 ? nb : std::min(ctas, nb);
         }
-        const size_t grid = static_cast<size_t>(sms) * b->resident_ctas[variant][ni ? 1 : 0][1];
-        b->lists.push_back({variant, limiter, ni, static_cast<int>(work.size()), kv.second.count});
+        ctas = std::max(1, ctas);
+        const size_t grid = static_cast<size_t>(sms) * ctas;
+        b->lists.push_back({variant, limiter, ni, static_cast<int>(work.size()), kv.second.count, ctas});
         // The CTAs walk a list with a grid stride. Highest items first, and every second round of
         // the grid in reverse (counted from the last, which may be partial), so that a CTA with a
         // high item in one round has a low one, or none, in the next. In list order 15 of 2383
@@ -568,8 +569,7 @@ void launch_step(mhdb_batch* b, int sms)
         for (const auto& l : b->lists) {
             auto fn = batch_fn<Policy>(l.variant, l.limiter, l.ni, stage);
             const size_t sm = K::smem(l.variant, l.ni, stage);
-            const int grid =
-                std::min(l.count, sms * b->resident_ctas[l.variant][l.ni ? 1 : 0][stage - 1]);
+            const int grid = std::min(l.count, sms * l.ctas);
             fn<<<grid, K::variant(l.variant).threads, sm, b->stream>>>(descs, b->work + l.offset,
                                                                       l.count);
             ++b->launches;
