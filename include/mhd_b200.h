@@ -217,6 +217,11 @@ int mhdb_set_tile_config(mhdb_solver* h, int config);
    counterpart (the reference has no bulk copies). */
 int mhdb_debug_stall_copies(mhdb_solver* h, int extra_bytes);
 
+/* Additive, for tests: rows (1 to 64, at most the configuration's tile height) of the strip marches'
+   segments in place of the choice by the grid's size, so that small grids reach the marches' row
+   loop. 0 (the default) restores the choice. Other kernels are unaffected. */
+int mhdb_debug_segment_rows(mhdb_solver* h, int rows);
+
 /* ---------------------------------------------------------------- strips of one grid (additive)
 
    One grid split into y strips, one solver per strip (on one GPU or on several): each strip's

@@ -33,7 +33,7 @@ EXPORTS = (
     "mhdb_batch_launch", "mhdb_batch_poll", "mhdb_batch_config_count", "mhdb_batch_config_info",
     "mhdb_batch_set_config", "mhdb_set_cell_size", "mhdb_set_reduce_rows", "mhdb_strip_view", "mhdb_strip_begin",
     "mhdb_strip_step", "mhdb_strip_finish", "mhdb_strip_poll", "mhdb_strip_end",
-    "mhdb_debug_stall_copies", "mhdb_batch_debug_stall_copies", "mhdb_configure_shapes",
+    "mhdb_debug_stall_copies", "mhdb_debug_segment_rows", "mhdb_batch_debug_stall_copies", "mhdb_configure_shapes",
     "mhdb_get_mask",
 )
 
@@ -123,6 +123,7 @@ def _load() -> C.CDLL:
         "mhdb_tile_config_kind": ([C.c_int, C.c_int], C.c_int),
         "mhdb_set_tile_config": ([h, C.c_int], C.c_int),
         "mhdb_debug_stall_copies": ([h, C.c_int], C.c_int),
+        "mhdb_debug_segment_rows": ([h, C.c_int], C.c_int),
         "mhdb_configure_shapes": ([h, C.c_int, C.c_int, C.POINTER(Shape), C.c_int, C.c_int],
                                   C.c_int),
         "mhdb_get_mask": ([h, C.POINTER(C.c_uint8), C.c_size_t], C.c_int),
@@ -331,6 +332,11 @@ class DeviceSolver:
         """Test hook: make one bulk-copy wait of the TMA strip marches run out
         (mhdb_debug_stall_copies); 0 turns it off."""
         raise_for(lib.mhdb_debug_stall_copies(self._h, int(extra_bytes)), self._h)
+
+    def debug_segment_rows(self, rows: int) -> None:
+        """Test hook: rows of the strip marches' segments (mhdb_debug_segment_rows); 0 restores the
+        choice by the grid's size."""
+        raise_for(lib.mhdb_debug_segment_rows(self._h, int(rows)), self._h)
 
     # Deferred solves of one strip of a split grid (strips.py drives them).
     def set_cell_size(self, dx: float, dy: float) -> None:

@@ -251,6 +251,7 @@ struct mhdb_solver {
 
     int tile_config = -1; // index into the compiled tile configurations (-1: by grid size)
     int stall_tx = 0;     // test hook of the bounded copy waits (mhdb_debug_stall_copies)
+    int segment_rows = 0; // test hook of the strip marches' segments (mhdb_debug_segment_rows)
     bool profiling = false;
     std::vector<Prof> prof_pending;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_pool;
@@ -496,9 +497,12 @@ StepPlan make_plan(mhdb_solver* h, const mhdb_params* p)
     if (sk.threads == 0) {
         throw ApiError{MHDB_INVALID_ARGUMENT, "no stage kernel for this configuration"};
     }
-    const int rows = sk.segments ? segment_rows(h->grid.nx, h->grid.ny, sk.tile_x, sk.tile_y,
-                                          h->sms * sk.min_blocks)
-                           : sk.tile_y;
+    int rows = sk.tile_y;
+    if (sk.segments) {
+        rows = h->segment_rows > 0 ? std::min(h->segment_rows, sk.tile_y)
+                                   : segment_rows(h->grid.nx, h->grid.ny, sk.tile_x, sk.tile_y,
+                                                  h->sms * sk.min_blocks);
+    }
     s.a1.rows = s.a2.rows = s.b1.rows = s.b2.rows = rows;
     for (int q = 0; q < 2; ++q) {
         s.c1[q].rows = s.c2[q].rows = rows;
@@ -605,7 +609,7 @@ std::vector<double> plan_key(const mhdb_solver* h, const mhdb_params* p, const S
             static_cast<double>(h->tile_config),
             h->grid.x_min, h->grid.x_max, h->grid.y_min, h->grid.y_max, h->dx, h->dy,
             static_cast<double>(h->geom.ry0), static_cast<double>(h->geom.ry1),
-            static_cast<double>(h->stall_tx)};
+            static_cast<double>(h->stall_tx), static_cast<double>(h->segment_rows)};
 }
 
 void launch_steps(mhdb_solver* h, const mhdb_params* p, const StepPlan& s, int n)
@@ -1322,6 +1326,19 @@ int mhdb_debug_stall_copies(mhdb_solver* h, int extra_bytes)
         return MHDB_INVALID_ARGUMENT;
     }
     h->stall_tx = extra_bytes;
+    return MHDB_OK;
+}
+
+int mhdb_debug_segment_rows(mhdb_solver* h, int rows)
+{
+    if (h == nullptr) {
+        return MHDB_INVALID_ARGUMENT;
+    }
+    if (rows < 0 || rows > 64) {
+        h->last_error = "segment rows must lie in [0, 64]";
+        return MHDB_INVALID_ARGUMENT;
+    }
+    h->segment_rows = rows;
     return MHDB_OK;
 }
 
