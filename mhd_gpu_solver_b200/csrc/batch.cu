@@ -256,8 +256,8 @@ struct BatchKernels<PolicyMixed> {
         if (v == 3) return {kMarchOwned, 32, 32, MHDB_KERNEL_MARCH_TMA_DELTA};
         return {kMarchOwned, 32, 32, MHDB_KERNEL_MARCH_TMA};
     }
-    // The increment form from 128^2 cells up; smaller solves keep U* as a hi + lo pair (TMA march of
-    // the stored form; the increment form's error against FP64 is about a tenth larger), in a list
+    // The increment form from 128^2 cells up; smaller solves store U* (TMA march of the stored form;
+    // the increment form's error against FP64 is about a tenth larger, kernels_mixed.cu), in a list
     // and launches of their own: in the increment form's list 16 solves of sides 64-1024 took 348 us
     // per step, this way 389, 64 of them 1000 and 1035, 64 solves of 64^2 alone 82 and 55. As the
     // default before, configuration 1 needs 407, 1054 and 53.

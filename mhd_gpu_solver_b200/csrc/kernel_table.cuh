@@ -123,7 +123,7 @@ void fill_pair(StageKernels& k)
         k.tile_x = Cfg::NW * kMarchOwned;
         k.tile_y = Cfg::LY;
         k.segments = true;
-        k.min_blocks = E == 8 && Cfg::NW == 1 && Cfg::MINB == 10 ? 12 : Cfg::MINB; // 168 registers fit 12
+        k.min_blocks = E == 8 && Cfg::NW == 1 && Cfg::MINB == 10 ? 12 : Cfg::MINB; // the 168 registers of a request for 10 fit 12
         k.threads = Cfg::NW * 32;
         k.smem = march_tma_smem_bytes<1, Cfg::ST1, E, (K > 0 ? 1 : 0)>(Cfg::NW);
         k.smem2 = march_tma_smem_bytes<2, Cfg::ST2, E, K>(Cfg::NW);

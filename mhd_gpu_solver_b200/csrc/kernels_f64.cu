@@ -28,8 +28,9 @@ int stage_config_count_f64() { return kCount; }
 // latencies, the one-warp register march (configuration 8), above the TMA march (configuration 7).
 // Per step, tile kernel (configuration 2) / register / TMA march: 128^2 15.8 / 14.0 / 15.1 us, 256^2
 // 23.3 / 24.1 / 25.7, 300x173 23.7 / 20.9 / 21.4, 400^2 48.9 / 37.9 / 38.6, 512^2 67 / 52.4 / 51.1,
-// 1024^2 258 / 204 / 162. Masked grids march from 1200^2 cells up and run the tile kernel
-// (configuration 0) below: 512^2 83 against 105 us, 1024^2 304 and 313, 1448^2 594 and 506.
+// 1024^2 258 / 204 / 162 (at 256^2 the tile kernel's blocks fill exactly one wave). Masked grids
+// march from 1200^2 cells up and run the tile kernel (configuration 0) below: 512^2 83 against 105
+// us, 1024^2 304 and 313, 1448^2 594 and 506.
 int default_stage_config_f64(long long cells, bool mask)
 {
     if (mask) {

@@ -46,9 +46,10 @@ int stage_config_count_mixed() { return kCount; }
 // copies to set up (per step, register against TMA march: 128^2 13.7 and 15.2 us, 301x173 17.1 and
 // 19.2, 400^2 26.6 and 29.6, 512^2 38 and 40, 640^2 49 and 50, 724^2 56 and 56; the tile kernel took
 // 18.5, 21.5, 36, 46 and 168 us at 128^2, 301x173, 400^2, 512^2 and 1024^2). From 724^2 up the TMA
-// march is the faster one (900^2 90 and 84 us, 1024^2 110 and 99), but the increment form rounds
-// U* - U^n to FP32 where the stored form keeps U* as a hi + lo pair, and its error against FP64 is 10
-// to 16 % larger (800x760: 2.9e-8 against 2.6e-8), so it serves only the sizes it was chosen for.
+// march is the faster one (900^2 90 and 84 us, 1024^2 110 and 99), but the increment form's stage 2
+// reads U* as fl(hi(U^n) + delta), rounded twice where the stored hi plane is rounded once, and its
+// error against FP64 is 10 to 16 % larger (800x760: 2.9e-8 against 2.6e-8), so it serves only the
+// sizes it was chosen for.
 // Masked grids of at least 1024^2 cells run the stored-form TMA march (configuration 11), smaller
 // ones the tile kernel: the march stores a solid cell from the row's FP32 primitives, the tile kernel
 // from the FP64 wall fill, so the march stays with the sizes it was chosen for (512^2 74 against 68

@@ -182,7 +182,7 @@ __device__ __forceinline__ double march_tma_strip(const typename Policy::Args& a
     // Mask byte of this lane's cell of row y: 0 for a solid interior cell, non-zero for a fluid one and
     // for ghosts. FP32 loads each byte once, a row before its primitives are formed, and keeps it
     // until the cell's update two rows later, instead of waiting for global memory twice a row
-    // (masked non-ideal 2048^2 step 585 -> 574 us). FP64 has no registers for it (5 % slower) and
+    // (masked non-ideal 2048^2: 1 % of a step, 15.12 -> 14.97 ms per 25). FP64 has no registers for it (5 % slower) and
     // reads the mask where it is used.
     auto mask_byte = [&](int y) -> int {
         if constexpr (MASK && sizeof(T) == 4) {

@@ -178,7 +178,7 @@ int mhdb_solve_steps_noalloc_f64(const mhdb_grid* grid, int bc_x, int bc_y,
 
     // The register march (configuration 8), a handle's choice for most grids within the limit: unlike
     // the bulk copies of the TMA march it takes the caller's dense planes with any row pitch and base
-    // alignment (321x257, 50 steps: 2.24 ms with the tile kernel, 1.44 ms).
+    // alignment (321x257, 50 steps: 2.24 ms with the tile kernel, 1.48 ms).
     const StageKernels sk = select_stage_f64(params->limiter, k.ni_any != 0, false, 8);
     if (sk.threads == 0) {
         return fail(MHDB_INVALID_ARGUMENT, "no stage kernel for this configuration");

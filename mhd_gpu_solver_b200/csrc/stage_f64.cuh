@@ -64,7 +64,7 @@ struct StageArgsF64 {
     Geometry geom;
     Consts k;
     int walls;           // reflective wall fill of solid cells
-    int rows;            // rows of a warp's segment (TMA strip marches)
+    int rows;            // rows of a warp's segment (strip marches)
 };
 
 struct PolicyF64 {

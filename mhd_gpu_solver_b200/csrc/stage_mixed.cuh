@@ -36,7 +36,7 @@ struct StageArgsMx {
     Geometry geom;
     Consts k;
     int walls;
-    int rows;            // rows of a warp's segment (TMA strip marches)
+    int rows;            // rows of a warp's segment (strip marches)
 };
 
 // One state buffer of 9 * plane * 8 bytes viewed as 9 hi planes followed by 9 lo planes.

@@ -22,7 +22,8 @@ NONIDEAL = dict(ohmic=True, hall=True, ambipolar=True, eta_ohm=1e-3, eta_hall=1e
 def test_default_keeps_the_intermediate_state_as_a_pair(nx, ny, nonideal):
     """Below 1024^2 cells the default stores U* as hi + lo pairs, as the tile kernel (configuration 0)
     does. The two kernels do the same FP32 operations with other contractions, so their errors agree
-    to a few in a thousand; an increment rounded to FP32 would add 10 to 16 %. Held to 2 %."""
+    to a few in a thousand; the increment form, whose stage 2 reads U* rounded twice, adds 10 to 16 %.
+    Held to 2 %."""
     U0 = initial_state(wl.fourier_state(nx, ny, 3), 5.0 / 3.0)
     p = orc.Params(limiter=orc.VANLEER, max_steps=6, fixed_steps=True,
                    **(NONIDEAL if nonideal else {}))
